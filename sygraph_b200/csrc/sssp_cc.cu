@@ -745,16 +745,30 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A parent as this SM last saw it.  The giant component's root is where most
+// walks end, and one address read from the L2 by every thread serves about
+// one read a cycle; from the L1 it costs nothing.  Parents only ever move to
+// ancestors, so an old value is an ancestor too.
+__device__ __forceinline__ uint32_t ld_seen(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.cta.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
   for (;;) {
-    const uint32_t p = ld_relaxed(parent + x);
+    const uint32_t p = ld_seen(parent + x);
     if (p == x) return x;
-    const uint32_t gp = ld_relaxed(parent + p);
+    const uint32_t gp = ld_seen(parent + p);
     if (gp != p) st_relaxed(parent + x, gp);  // path halving: gp is an ancestor of x
     x = gp;
   }
 }
 
+// Both walks may end on a vertex that has been linked since: linking the
+// larger under such a one still joins the two trees (ids fall along every
+// link, so it makes no cycle), and a CAS on one fails and hands over its
+// parent, from which the walk goes on -- strictly down, so it ends.
 __device__ __forceinline__ void uf_unite(uint32_t* parent, uint32_t u, uint32_t v) {
   for (;;) {
     u = uf_find(parent, u);
@@ -765,105 +779,202 @@ __device__ __forceinline__ void uf_unite(uint32_t* parent, uint32_t u, uint32_t 
       u = v;
       v = t;
     }
-    if (atomicCAS(parent + u, u, v) == u) return;  // larger root under the smaller
+    const uint32_t old = atomicCAS(parent + u, u, v);  // larger root under the smaller
+    if (old == u) return;
+    u = old;
   }
 }
 
-__global__ void __launch_bounds__(256) uf_init_kernel(uint32_t* __restrict__ parent, uint32_t* __restrict__ top,
-                                                      uint32_t n) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    parent[v] = v;
-    top[v] = v;
+// State of one union-find run, on the device.
+struct UfState {
+  unsigned long long big;  // list of long rows: (entries << 32) | chunks
+  uint32_t giant;          // root of the largest sampled component
+  uint32_t again;          // another sampled neighbour per vertex is worth it
+};
+
+struct UfParams {
+  const uint32_t* ro;
+  const uint32_t* col;
+  uint32_t n;
+  uint32_t* parent;  // the labels, at the end
+  uint32_t* top;     // n: per root, the largest id of its tree
+  uint32_t* list;    // n: long rows outside the giant component
+  uint32_t* list_start;  // n: their first chunks
+  UfState* st;
+  unsigned long long* result;
+  GridBarrier* bar;
+};
+
+constexpr uint32_t kUfThreads = 1024, kUfSamples = kUfThreads;
+// Sampled neighbours after the first, at most.  On shuffled grids each round
+// halves the trees and the giant component appears with the sixth (1700^2:
+// 1.31 ms with three rounds, 0.38 with six); RMAT needs none or one, uniform
+// random graphs two or three.
+constexpr uint32_t kUfRounds = 6;
+constexpr uint32_t kUfBig = 1024;  // edges per chunk of a long row
+
+// The root of v in a forest whose roots stay: parent[v] moves up on the way.
+// Only v's thread writes parent[v] here, and every value it takes is an
+// ancestor, so a long chain (a column of a grid) halves for the threads
+// behind it -- once they read what others wrote, so a walk of more than four
+// steps goes on from the L2.
+__device__ __forceinline__ uint32_t uf_flatten(uint32_t* parent, uint32_t v) {
+  uint32_t p = ld_seen(parent + v);
+  if (p == v) return v;
+  for (uint32_t step = 0;; step++) {
+    const uint32_t gp = step < 4 ? ld_seen(parent + p) : ld_relaxed(parent + p);
+    if (gp == p) return p;  // a root stays one here, whenever it was read
+    st_relaxed(parent + v, gp);
+    p = gp;
   }
 }
 
-// Afforest-style order: every vertex first unites with its first kSampled
-// neighbours (one round per neighbour index; one round measured best on
-// RMAT-20 and RMAT-22, a second cost 18% on RMAT-22), the trees are
-// flattened, and
-// the root shared by most of 1024 sampled vertices is taken as the giant
-// component's; then only vertices outside it unite with their other
-// neighbours.  An edge skipped at an endpoint inside the giant component is
-// united from its other endpoint (the rows hold every edge both ways) unless
-// that endpoint is inside too.
-constexpr uint32_t kSampled = 1, kGiantSamples = 1024;
-
-__global__ void __launch_bounds__(256) uf_sample_kernel(const uint32_t* __restrict__ ro, const uint32_t* __restrict__ col,
-                                                        uint32_t n, uint32_t r, uint32_t* parent) {
-  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-    const uint32_t b = ro[u];
-    if (ro[u + 1] - b > r) uf_unite(parent, u, col[b + r]);
-  }
-}
-
-// One block of kGiantSamples threads: the most frequent root among the
-// samples (ties to the larger id); the trees are flat when it runs.
-__global__ void __launch_bounds__(kGiantSamples) uf_giant_kernel(const uint32_t* parent, uint32_t n,
-                                                                 uint32_t* __restrict__ giant) {
-  __shared__ uint32_t s_root[kGiantSamples];
+// Block 0, on flat trees: the root that most of 1024 sampled vertices with
+// edges share (vertices without edges are components of their own whatever is
+// linked), and whether another round is worth it: while that root holds less
+// than three quarters of the samples.  Each warp offers the most frequent
+// root of its 32 samples and counts the root that one warp offers over all
+// samples.  The choice only steers the work.
+__device__ __forceinline__ void uf_pick_giant(const UfParams& P) {
+  __shared__ uint32_t s_root[kUfSamples], s_offer[32];
   __shared__ unsigned long long s_best;
-  const uint32_t i = threadIdx.x;
-  s_root[i] = ld_relaxed(parent + (uint32_t)(((uint64_t)i * 2654435761u) % n));
+  const uint32_t i = threadIdx.x, lane = i & 31u, warp = i >> 5;
+  const uint32_t v = (uint32_t)(((uint64_t)i * 2654435761u) % P.n);
+  const bool has = P.ro[v] < P.ro[v + 1];
+  const uint32_t r = has ? ld_relaxed(P.parent + v) : 0xffffffffu;
+  s_root[i] = r;
   if (i == 0) s_best = 0;
+  const uint32_t c = has ? (uint32_t)__popc(__match_any_sync(__activemask(), r)) : 0u;
+  __syncwarp();
+  const uint32_t best = __reduce_max_sync(kFullMask, c);
+  const uint32_t first = __ffs(__ballot_sync(kFullMask, c == best)) - 1u;
+  if (lane == first) s_offer[warp] = r;
+  const uint32_t samples = __syncthreads_count(has);
+  const uint32_t mine = s_offer[warp];
+  uint32_t k = 0;
+  for (uint32_t j = lane; j < kUfSamples; j += 32) k += s_root[j] == mine;
+  k = sygraph::detail::warp_sum(k);
+  if (lane == 0 && mine != 0xffffffffu) atomicMax(&s_best, ((unsigned long long)k << 32) | mine);
   __syncthreads();
-  uint32_t c = 0;
-  for (uint32_t j = 0; j < kGiantSamples; j++) c += s_root[j] == s_root[i];
-  atomicMax(&s_best, ((unsigned long long)c << 32) | s_root[i]);
-  __syncthreads();
-  if (i == 0) *giant = (uint32_t)s_best;
-}
-
-__global__ void __launch_bounds__(256) uf_rest_kernel(const uint32_t* __restrict__ ro, const uint32_t* __restrict__ col,
-                                                      uint32_t n, const uint32_t* __restrict__ giant, uint32_t* parent) {
-  const uint32_t g = *giant;
-  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-    if (ld_relaxed(parent + u) == g) continue;
-    const uint32_t e = ro[u + 1];
-    for (uint32_t i = ro[u] + kSampled; i < e; i++) uf_unite(parent, u, col[i]);
+  if (i == 0) {
+    P.st->giant = samples ? (uint32_t)s_best : 0xffffffffu;
+    P.st->again = 4 * (uint32_t)(s_best >> 32) < 3 * samples;
   }
 }
 
-// Flattening: every vertex's parent becomes its root.  The walk only reads:
-// a path-halving store here could land after another vertex's root and
-// replace it with an ancestor short of the root.  The only stores are roots,
-// so every value read is still an ancestor.
-__global__ void __launch_bounds__(256) uf_flatten_kernel(uint32_t* parent, uint32_t n) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-    uint32_t x = v;
-    for (uint32_t p = ld_relaxed(parent + x); p != x; p = ld_relaxed(parent + x)) x = p;
-    st_relaxed(parent + v, x);
-  }
-}
-
-// top[root] = largest id of the root's (flat) tree: one atomicMax per root
-// and warp, and for the giant component's root one per block (through
-// shared memory), since most vertices carry it.
-__global__ void __launch_bounds__(256) uf_top_kernel(const uint32_t* __restrict__ parent, uint32_t* top, uint32_t n,
-                                                     const uint32_t* __restrict__ giant) {
+// Connected components, one cooperative launch:
+//   hook   every vertex hooks onto its first neighbour when that has the
+//          smaller id.  Ids fall along every link, so the links form a forest
+//          without a find or a CAS
+//   link   while no giant component shows (and at most kUfRounds times), a
+//          further neighbour per vertex outside the largest one: the larger
+//          of the two flat trees' roots hooks onto the smallest one that any
+//          of its edges offers; an edge that loses is left to the rest pass.
+//          One atomicMin per distinct root of a warp that still improves
+//   rest   every edge of the vertices outside the giant component is united
+//          (a CAS on the root).  An edge skipped at an endpoint inside the
+//          giant component is united from its other endpoint (the rows hold
+//          every edge both ways) unless that one is inside too.  A warp ranks
+//          the edges of 32 vertices across its lanes; rows of kUfBig edges or
+//          more are cut in chunks for the whole grid
+//   top    trees flattened, and the largest id of each tree at its root
+//   label  every vertex takes its root's largest id
+// What bounds it is one random access per vertex and phase and, before, the
+// roots: RMAT of 3.0 M vertices with shuffled ids took 153 ms when a hub that
+// the sampled links had missed was one thread's work, 0.92 ms with its rows
+// cut but a find and a CAS per sampled edge (all of them end on one address
+// in the L2), 0.27 ms in this form; RMAT-22 0.42 ms -> 0.17 ms.  The phases are
+// one launch because the rounds that a graph does not need cost nothing there
+// (nine empty launches are 20 us, a third of the time on RMAT-10).
+__global__ void __launch_bounds__(kUfThreads, 2) uf_kernel(UfParams P) {
   __shared__ uint32_t s_giant_max;
-  const uint32_t lane = threadIdx.x & 31u, gr = *giant;
+  const uint32_t lane = threadIdx.x & 31u, n = P.n;
+  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  const uint32_t *ro = P.ro, *col = P.col;
+  uint32_t* parent = P.parent;
+  if (gtid == 0) P.st->big = 0;
   if (threadIdx.x == 0) s_giant_max = 0;
-  __syncthreads();
-  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < n; base += gridDim.x * blockDim.x) {
+  for (uint32_t v = gtid; v < n; v += nthreads) {
+    const uint32_t b = ro[v], e = ro[v + 1];
+    st_relaxed(parent + v, b < e ? min(v, col[b]) : v);
+    P.top[v] = v;
+  }
+  if (!grid_sync(P.bar)) return;
+  uint32_t g;
+  for (uint32_t round = 0;; round++) {
+    for (uint32_t v = gtid; v < n; v += nthreads) uf_flatten(parent, v);
+    if (!grid_sync(P.bar)) return;
+    if (blockIdx.x == 0) uf_pick_giant(P);
+    if (!grid_sync(P.bar)) return;
+    g = ld_relaxed(&P.st->giant);
+    if (round == kUfRounds || !ld_relaxed(&P.st->again)) break;
+    for (uint32_t u = gtid; u < n; u += nthreads) {
+      const uint32_t pu = ld_seen(parent + u);
+      if (pu == g) continue;
+      const uint32_t b = ro[u], e = ro[u + 1];
+      if (b == e) continue;
+      // the row's last edge, its middle, its first quarter, its first edge
+      const uint32_t q = round & 3u;
+      const uint32_t at = q == 0 ? e - 1 : q == 1 ? b + (e - b) / 2 : q == 2 ? b + (e - b) / 4 : b;
+      const uint32_t pw = ld_seen(parent + col[at]);
+      if (pu == pw) continue;
+      const uint32_t hi = max(pu, pw), lo = min(pu, pw);
+      const uint32_t same = __match_any_sync(__activemask(), hi);
+      const uint32_t mn = __reduce_min_sync(same, lo);
+      if (lane == __ffs(same) - 1u && mn < ld_seen(parent + hi)) atomicMin(parent + hi, mn);
+    }
+    if (!grid_sync(P.bar)) return;
+  }
+  for (uint32_t base = gtid - lane; base < n; base += nthreads) {
+    const uint32_t u = base + lane;
+    const bool open = u < n && ld_seen(parent + u) != g;
+    if (!__any_sync(kFullMask, open)) continue;
+    const uint32_t b = open ? ro[u] : 0u;
+    uint32_t d = open ? ro[u + 1] - b : 0u;
+    if (d >= kUfBig) {
+      const uint32_t chunks = (d - 1) / kUfBig + 1;
+      const unsigned long long old = atomicAdd(&P.st->big, (1ull << 32) | chunks);
+      P.list[(uint32_t)(old >> 32)] = u;
+      P.list_start[(uint32_t)(old >> 32)] = (uint32_t)old;
+      d = 0;
+    }
+    const uint32_t incl = warp_inclusive_scan(d);
+    const uint32_t total = __shfl_sync(kFullMask, incl, 31), excl = incl - d;
+    for (uint32_t r0 = 0; r0 < total; r0 += 32) {
+      const uint32_t r = r0 + lane;
+      const uint32_t o = warp_owner_of_rank(incl, min(r, total - 1));
+      const uint32_t ob = __shfl_sync(kFullMask, b, o), oe = __shfl_sync(kFullMask, excl, o);
+      if (r < total) uf_unite(parent, base + o, col[ob + (r - oe)]);
+    }
+  }
+  if (!grid_sync(P.bar)) return;
+  const unsigned long long big = ld_cg(&P.st->big);
+  for (uint32_t c = gtid >> 5; c < (uint32_t)big; c += nthreads >> 5) {
+    const uint32_t o = warp_find_owner(P.list_start, (uint32_t)(big >> 32), c);
+    const uint32_t u = ld_cg(P.list + o), b = ro[u] + (c - ld_cg(P.list_start + o)) * kUfBig;
+    const uint32_t e = b + min(ro[u + 1] - b, kUfBig);
+    for (uint32_t i = b + lane; i < e; i += 32) uf_unite(parent, u, col[i]);
+  }
+  if (big && !grid_sync(P.bar)) return;
+  // one atomicMax per root and warp, and for the giant component's root, which
+  // most vertices carry, one per block (through shared memory)
+  for (uint32_t base = gtid - lane; base < n; base += nthreads) {
     const uint32_t v = base + lane;
     const bool ok = v < n;
-    const uint32_t r = ok ? parent[v] : 0xffffffffu;
-    const uint32_t same = __match_any_sync(0xffffffffu, r);
-    const uint32_t mx = __reduce_max_sync(same, ok ? v : 0u);
-    if (ok && lane == __ffs(same) - 1u) {
-      if (r == gr)
-        atomicMax(&s_giant_max, mx);
-      else
-        atomicMax(top + r, mx);
+    const uint32_t r = ok ? uf_flatten(parent, v) : 0xffffffffu;
+    const uint32_t in_giant = __reduce_max_sync(kFullMask, ok && r == g ? v + 1 : 0u);
+    if (lane == 0 && in_giant) atomicMax(&s_giant_max, in_giant);
+    if (ok && r != g && r != v) {
+      const uint32_t same = __match_any_sync(__activemask(), r);
+      const uint32_t mx = __reduce_max_sync(same, v);
+      if (lane == __ffs(same) - 1u) atomicMax(P.top + r, mx);
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && s_giant_max) atomicMax(top + gr, s_giant_max);
-}
-
-// labels[v] = top[root(v)]; in place: each thread reads only its own parent.
-__global__ void __launch_bounds__(256) uf_label_kernel(uint32_t* parent, const uint32_t* __restrict__ top, uint32_t n) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) parent[v] = top[parent[v]];
+  if (threadIdx.x == 0 && s_giant_max) atomicMax(P.top + g, s_giant_max - 1);
+  if (!grid_sync(P.bar)) return;
+  for (uint32_t v = gtid; v < n; v += nthreads) parent[v] = ld_cg(P.top + ld_cg(parent + v));
+  if (gtid == 0) P.result[0] = 1;  // one pass over the edges (most skipped)
 }
 
 }  // namespace
@@ -1343,21 +1454,12 @@ sg_status sg_cc_run_async(sg_cc_handle c) {
   const sg_graph g = c->g;
   c->used_union_find = c->method == SG_CC_UNION_FIND || (c->method == SG_CC_AUTO && !(g->flags & SG_GRAPH_DIRECTED));
   if (c->used_union_find) {
-    const unsigned vgrid = grid_for(g->n, 256, 8);
-    // scratch from the push workspace, idle on this path: the giant root in
-    // the first queue's first word, the per-root largest ids in the second
-    uint32_t *giant = c->ws.q.small, *top = c->ws.q.big;
-    uf_init_kernel<<<vgrid, 256, 0, c->stream>>>(c->labels, top, g->n);
-    for (uint32_t r = 0; r < kSampled; r++)
-      uf_sample_kernel<<<vgrid, 256, 0, c->stream>>>(g->fwd.ro, g->fwd.col, g->n, r, c->labels);
-    uf_flatten_kernel<<<vgrid, 256, 0, c->stream>>>(c->labels, g->n);
-    uf_giant_kernel<<<1, kGiantSamples, 0, c->stream>>>(c->labels, g->n, giant);
-    uf_rest_kernel<<<vgrid, 256, 0, c->stream>>>(g->fwd.ro, g->fwd.col, g->n, giant, c->labels);
-    uf_flatten_kernel<<<vgrid, 256, 0, c->stream>>>(c->labels, g->n);
-    uf_top_kernel<<<vgrid, 256, 0, c->stream>>>(c->labels, top, g->n, giant);
-    uf_label_kernel<<<vgrid, 256, 0, c->stream>>>(c->labels, top, g->n);
-    SG_CUDA(cudaGetLastError());
-    count_launch(6 + kSampled);
+    // scratch from the push workspace, idle on this path
+    static_assert(sizeof(UfState) <= 2 * sizeof(unsigned long long), "UfState lives in the last two result words");
+    SG_CUDA(cudaMemsetAsync(c->ws.bar, 0, sizeof(GridBarrier), c->stream));
+    UfParams P{g->fwd.ro, g->fwd.col, g->n, c->labels, c->ws.q.big, c->ws.q.small, c->ws.q.big_start,
+               reinterpret_cast<UfState*>(c->ws.result + 2), c->ws.result, c->ws.bar};
+    SG_TRY(launch_persistent(uf_kernel, P, 2, c->stream, (g->n - 1) / kUfThreads + 1, nullptr, kUfThreads));
   } else {
     SG_CUDA(cudaMemsetAsync(c->ws.bar, 0, sizeof(GridBarrier), c->stream));
     CcParams P{c->ws.loop(g), c->labels, c->ws.result};
@@ -1369,11 +1471,6 @@ sg_status sg_cc_run_async(sg_cc_handle c) {
 
 sg_status sg_cc_run(sg_cc_handle c, uint64_t* iterations) {
   SG_TRY(sg_cc_run_async(c));
-  if (c->used_union_find) {
-    SG_CUDA(cudaStreamSynchronize(c->stream));
-    if (iterations) *iterations = 1;  // one pass over the edges (most skipped)
-    return SG_OK;
-  }
   return c->ws.finish(c->stream, iterations);
 }
 

@@ -196,3 +196,32 @@ def test_cc_union_find_adversarial(sg, oracle, shape):
     for _ in range(2):
         cc.run()
         assert np.array_equal(cc.getLabels(), ref)
+
+
+@pytest.mark.parametrize("hub_degree", [1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("giant", ["dense", "sparse", "none"])
+def test_cc_union_find_hub_outside_giant(sg, oracle, hub_degree, giant):
+    """A star whose rows meet the long-row list (chunks of 1024 edges) while
+    the giant component is found at once, only after sampled rounds (a
+    shuffled grid), or not at all (paths of three)."""
+    rng = np.random.default_rng(hub_degree)
+    if giant == "dense":
+        g0 = sg.io.rmat(13)
+        s, d, n0 = np.repeat(np.arange(g0.n), np.diff(g0.row_offsets.astype(np.int64))), g0.column_indices, g0.n
+    elif giant == "sparse":
+        g0 = sg.io.grid(120, 0.0)
+        s, d, n0 = np.repeat(np.arange(g0.n), np.diff(g0.row_offsets.astype(np.int64))), g0.column_indices, g0.n
+    else:
+        n0 = 20000
+        s = np.array([v for v in range(n0 - 1) if v % 3 != 2])
+        d = s + 1
+    n = n0 + hub_degree + 1 + 5  # five vertices without edges
+    perm = rng.permutation(n)
+    s = np.concatenate([s, np.full(hub_degree, n0)])
+    d = np.concatenate([d, n0 + 1 + np.arange(hub_degree)])
+    g = sg.io.fromCOO(n, perm[s], perm[d], symmetrize=True, dedupe=True)
+    ref = oracle.cc_maxlabel(g)
+    cc = sg.algorithms.CC(sg.graph.build.fromCSR(g))
+    for _ in range(3):
+        cc.run()
+        assert np.array_equal(cc.getLabels(), ref)
