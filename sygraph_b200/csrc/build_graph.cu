@@ -3,17 +3,12 @@
 // io::csr::fromCOO (io/read_csr.hpp:260-300), formats::CSR::invert
 // (formats/csr.hpp:179-209) and the upload of GraphCSR
 // (graph/impls/graph_csr.hpp:394-426); sg_csr_from_edges is that host path.
-// Here one persistent cooperative kernel does it all:
-//   fill    entry 2i / 2i+1 (or i) = (u, v) / (v, u) of edge i as the key
-//           u * 2^b + v (2^b > n); a dropped entry (a self-loop when they are
-//           dropped, the reverse of a self-loop) gets the all-ones key, which
-//           sorts after every edge
-//   sort    LSD radix sort of (key, value) pairs, 8 bits per pass.  Each CTA
-//           owns one contiguous range of the array in every pass: it counts
-//           its digits, and after a grid barrier scatters its range in order,
-//           one thread per entry and 512 entries per round, equal digits
-//           ranked by warp match groups -- a stable sort, so equal keys keep
-//           their insertion order
+// Here:
+//   sort    entry 2i / 2i+1 (or i) = (u, v) / (v, u) of edge i as the key
+//           u * 2^b + v (2^b >= n), by a stable radix sort (radix_sort.cuh)
+//           whose first pass makes the entries from the edge list and leaves
+//           the dropped ones out (a self-loop when they are dropped, the
+//           reverse of a self-loop); equal keys keep their insertion order
 //   compact the first entry of every run of equal keys (every entry without
 //           de-duplication) is kept, in order: columns, values, and the row
 //           offset of each non-empty row; empty rows take the next row's
@@ -25,253 +20,176 @@
 #include <mutex>
 #include <vector>
 
-#include "engine_common.cuh"
+#include "radix_sort.cuh"
 
 namespace sgb {
 namespace gb {
 
-using namespace eng;
-using u64 = unsigned long long;
+using rsort::u64;
+using sygraph::detail::kFullMask;
 
-constexpr u64 kNone = ~0ull;
-constexpr uint32_t kWarps = kThreads / 32;
-
-struct BuildParams {
+// The entries of an edge list, in insertion order.
+struct EdgeSource {
   const uint32_t* src;
   const uint32_t* dst;
   const uint32_t* val;  // nullptr: every value is `one`
-  uint64_t count;
+  uint32_t entries;
   uint32_t n;
-  uint32_t b;  // bits per endpoint (2^b > n)
+  uint32_t b;  // bits per endpoint (2^b >= n)
   uint32_t one;
-  int symmetrize, dedupe, drop_self_loops;
-  uint64_t entries;
-  uint32_t passes;
-  u64* k0;
-  u64* k1;
-  uint32_t* v0;
-  uint32_t* v1;
-  uint32_t* hist;   // 256 * gridDim.x
-  u64* csum;        // gridDim.x
-  uint32_t* ro;     // n + 1
-  uint32_t* col;    // compacted columns (entries)
-  uint32_t* oval;   // compacted values (entries)
-  u64* m_out;
-  uint32_t* bad;    // an endpoint was >= n
-  GridBarrier* bar;
+  int symmetrize, drop_self_loops;
+  uint32_t* bad;  // an endpoint was >= n
+  __device__ __forceinline__ uint32_t size() const { return entries; }
+  __device__ __forceinline__ bool key_at(uint32_t i, u64* k) const {
+    const uint32_t j = symmetrize ? i >> 1 : i;
+    const bool rev = symmetrize && (i & 1u);
+    const uint32_t u = src[j], v = dst[j];
+    if (u >= n || v >= n) {
+      *bad = 1u;
+      return false;
+    }
+    *k = rev ? ((u64)v << b) | u : ((u64)u << b) | v;
+    return u != v || !(drop_self_loops || rev);
+  }
+  __device__ __forceinline__ uint32_t val_at(uint32_t i) const { return val ? val[symmetrize ? i >> 1 : i] : one; }
 };
 
-struct Shared {
-  uint32_t hist[256];
-  uint32_t base[256];
-  uint32_t tot[256];
-  uint32_t cnt[kWarps][256];
-  uint32_t scan[32];
-  uint32_t wmin[kWarps];
-  u64 red[32];
-};
+// Sorted keys are compacted in tiles, one bit per kept entry (the first of
+// its run of equal keys, or every entry without de-duplication).
+constexpr uint32_t kKeepThreads = 512, kKeepItems = 8, kKeepTile = kKeepThreads * kKeepItems;
 
-// Suffix minimum of x over the block's threads (thread t gets min of x over
-// t..blockDim-1).
-__device__ __forceinline__ uint32_t block_suffix_min(uint32_t x, Shared& S) {
+// Bit r: entry base + 32 r + lane is kept; `before`: the warp's kept entries
+// of the earlier lanes' and rounds' entries are counted by the caller.
+__device__ __forceinline__ uint32_t keep_bits(const u64* __restrict__ key, uint32_t count, int dedupe, uint64_t base) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (uint32_t r = 0; r < kKeepItems; r++) {
+    const uint64_t i = base + 32 * r;
+    if (i < count && (!dedupe || i == 0 || key[i - 1] != key[i])) bits |= 1u << r;
+  }
+  return bits;
+}
+
+__global__ void __launch_bounds__(kKeepThreads) keep_count_kernel(const u64* __restrict__ key, const uint32_t* count,
+                                                                  int dedupe, uint32_t* __restrict__ tile_kept) {
+  __shared__ uint32_t s_red[32];
+  const uint64_t base =
+      (uint64_t)blockIdx.x * kKeepTile + (threadIdx.x >> 5) * (32 * kKeepItems) + (threadIdx.x & 31u);
+  const uint32_t kept = sygraph::detail::block_sum<uint32_t>(__popc(keep_bits(key, *count, dedupe, base)), s_red);
+  if (threadIdx.x == 0) tile_kept[blockIdx.x] = kept;
+}
+
+__global__ void __launch_bounds__(kKeepThreads) keep_write_kernel(const u64* __restrict__ key,
+                                                                  const uint32_t* __restrict__ val,
+                                                                  const uint32_t* count, int dedupe, uint32_t b,
+                                                                  const uint32_t* __restrict__ tile_first,
+                                                                  const uint32_t* kept_total, uint32_t n,
+                                                                  uint32_t* __restrict__ ro, uint32_t* __restrict__ col,
+                                                                  uint32_t* __restrict__ oval) {
+  __shared__ uint32_t s_scan[32];
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t base = (uint64_t)blockIdx.x * kKeepTile + (threadIdx.x >> 5) * (32 * kKeepItems) + lane;
+  const uint32_t bits = keep_bits(key, *count, dedupe, base);
+  // kept entries before the warp's segment
+  const uint32_t mine = sygraph::detail::warp_sum(__popc(bits));
+  uint32_t all;
+  uint32_t pos = sygraph::detail::block_excl_scan(lane == 0 ? mine : 0u, &all, s_scan);
+  pos = tile_first[blockIdx.x] + __shfl_sync(kFullMask, pos, 0);
+#pragma unroll
+  for (uint32_t r = 0; r < kKeepItems; r++) {
+    const bool keep = (bits >> r) & 1u;
+    const uint32_t m = __ballot_sync(kFullMask, keep);
+    if (keep) {
+      const uint64_t i = base + 32 * r;
+      const uint32_t at = pos + __popc(m & ((1u << lane) - 1u));
+      const u64 k = key[i];
+      const uint32_t s = (uint32_t)(k >> b);
+      col[at] = (uint32_t)k & (uint32_t)((1ull << b) - 1u);
+      oval[at] = val[i];
+      // first kept entry of row s: nothing before it in the sorted order
+      // shares its row (a duplicate of the same key shares it and is not kept)
+      if (i == 0 || (uint32_t)(key[i - 1] >> b) != s) ro[s] = at;
+    }
+    pos += __popc(m);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) ro[n] = *kept_total;
+}
+
+// Rows without edges hold the all-ones word; they take the offset of the next
+// row that has some: a suffix minimum over ro[0, n] (ro[n] = m is set), by
+// tile minima, their suffix minima in one block, and the tiles again.
+__device__ __forceinline__ uint32_t block_suffix_min(uint32_t x, uint32_t* s_min) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const uint32_t y = __shfl_down_sync(kFullMask, x, d);
     if (lane + d < 32) x = min(x, y);
   }
-  if (lane == 0) S.wmin[warp] = x;
+  if (lane == 0) s_min[warp] = x;
   __syncthreads();
   uint32_t later = 0xffffffffu;
-  for (uint32_t w = warp + 1; w < nw; w++) later = min(later, S.wmin[w]);
+  for (uint32_t w = warp + 1; w < nw; w++) later = min(later, s_min[w]);
   __syncthreads();
   return min(x, later);
 }
 
-// LSD radix sort of (key, value) pairs, `passes` digits of 8 bits from bit
-// `shift0` up.  CTA c owns [lo, hi) of the array in every pass: it counts its
-// digits, and after a grid barrier scatters its range in order, one thread
-// per entry and blockDim entries per round, equal digits ranked by warp match
-// groups -- a stable sort.  On return kin / vin hold the sorted pairs (the
-// pointers are swapped after every pass).  False when a barrier wait ran out.
-__device__ __forceinline__ bool radix_sort_pairs(Shared& S, GridBarrier* bar, uint32_t* ghist, u64*& kin,
-                                                 u64*& kout, uint32_t*& vin, uint32_t*& vout, uint64_t lo,
-                                                 uint64_t hi, uint32_t shift0, uint32_t passes) {
-  const uint32_t G = gridDim.x, c = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (uint32_t p = 0; p < passes; p++) {
-    const uint32_t sh = shift0 + 8 * p;
-    if (t < 256) S.hist[t] = 0;
-    __syncthreads();
-    for (uint64_t i = lo + t; i < hi; i += blockDim.x) atomicAdd(&S.hist[(uint32_t)(kin[i] >> sh) & 255u], 1u);
-    __syncthreads();
-    if (t < 256) ghist[(size_t)t * G + c] = S.hist[t];
-    if (!grid_sync(bar)) return false;
-    uint32_t tot = 0, before = 0;
-    if (t < 256) {
-      for (uint32_t cc = 0; cc < G; cc++) {
-        const uint32_t x = ld_cg(ghist + (size_t)t * G + cc);
-        tot += x;
-        if (cc < c) before += x;
-      }
-    }
-    uint32_t all;
-    const uint32_t dbase = sygraph::detail::block_excl_scan(t < 256 ? tot : 0u, &all, S.scan);
-    if (t < 256) S.base[t] = dbase + before;
-    __syncthreads();
-    for (uint64_t r0 = lo; r0 < hi; r0 += blockDim.x) {
-      const uint64_t i = r0 + t;
-      const bool in = i < hi;
-      const u64 k = in ? kin[i] : 0ull;
-      const uint32_t vv = in ? vin[i] : 0u;
-      const uint32_t d = in ? ((uint32_t)(k >> sh) & 255u) : 256u;
-      for (uint32_t x = t; x < kWarps * 256; x += blockDim.x) (&S.cnt[0][0])[x] = 0u;
-      __syncthreads();
-      const uint32_t grp = __match_any_sync(kFullMask, d);
-      const uint32_t rank = __popc(grp & ((1u << lane) - 1u));
-      if (in && rank == 0) S.cnt[warp][d] = __popc(grp);
-      __syncthreads();
-      if (t < 256) {
-        uint32_t run = 0;
-        for (uint32_t w = 0; w < kWarps; w++) {
-          const uint32_t x = S.cnt[w][t];
-          S.cnt[w][t] = run;
-          run += x;
-        }
-        S.tot[t] = run;
-      }
-      __syncthreads();
-      if (in) {
-        const uint32_t pos = S.base[d] + S.cnt[warp][d] + rank;
-        kout[pos] = k;
-        vout[pos] = vv;
-      }
-      __syncthreads();
-      if (t < 256) S.base[t] += S.tot[t];
-    }
-    u64* tk = kin;
-    kin = kout;
-    kout = tk;
-    uint32_t* tv = vin;
-    vin = vout;
-    vout = tv;
-    if (!grid_sync(bar)) return false;
-  }
-  return true;
-}
-
-__global__ void __launch_bounds__(kThreads, 2) build_kernel(BuildParams P) {
-  __shared__ Shared S;
-  const uint32_t G = gridDim.x, c = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const uint64_t nth = (uint64_t)G * blockDim.x;
-  const uint64_t gtid = (uint64_t)c * blockDim.x + t;
-  const uint64_t E = P.entries;
-  const uint64_t per = (E + G - 1) / G;
-  const uint64_t lo = min(E, (uint64_t)c * per), hi = min(E, lo + per);
-  const uint32_t bmask = (1u << P.b) - 1u;
-
-  // ---- fill
-  for (uint64_t i = gtid; i < E; i += nth) {
-    const uint64_t j = P.symmetrize ? i >> 1 : i;
-    const bool rev = P.symmetrize && (i & 1);
-    const uint32_t u = P.src[j], v = P.dst[j];
-    bool drop = (P.drop_self_loops && u == v) || (rev && u == v);
-    if (u >= P.n || v >= P.n) {
-      atomicOr(P.bad, 1u);
-      drop = true;
-    }
-    const uint32_t a = rev ? v : u, z = rev ? u : v;
-    P.k0[i] = drop ? kNone : (((u64)a << P.b) | z);
-    P.v0[i] = P.val ? P.val[j] : P.one;
-  }
-  for (uint64_t v = gtid; v <= P.n; v += nth) P.ro[v] = 0xffffffffu;
-  if (!grid_sync(P.bar)) return;
-
-  // ---- sort
-  u64* kin = P.k0;
-  u64* kout = P.k1;
-  uint32_t* vin = P.v0;
-  uint32_t* vout = P.v1;
-  if (!radix_sort_pairs(S, P.bar, P.hist, kin, kout, vin, vout, lo, hi, 0, P.passes)) return;
-
-  // ---- compact: kept entries in order, and the row start of each non-empty row
-  auto keep = [&](uint64_t i, u64 k) {
-    return k != kNone && (!P.dedupe || i == 0 || kin[i - 1] != k);
-  };
-  u64 mine = 0;
-  for (uint64_t i = lo + t; i < hi; i += blockDim.x) mine += keep(i, kin[i]) ? 1u : 0u;
-  const u64 csum = sygraph::detail::block_sum<u64>(mine, S.red);
-  if (t == 0) P.csum[c] = csum;
-  if (!grid_sync(P.bar)) return;
-  u64 base = 0, m = 0;
-  for (uint32_t cc = 0; cc < G; cc++) {
-    const u64 x = ld_cg(P.csum + cc);
-    m += x;
-    if (cc < c) base += x;
-  }
-  for (uint64_t r0 = lo; r0 < hi; r0 += blockDim.x) {
-    const uint64_t i = r0 + t;
-    const u64 k = i < hi ? kin[i] : kNone;
-    const bool kp = i < hi && keep(i, k);
-    uint32_t total;
-    const uint32_t ex = sygraph::detail::block_excl_scan(kp ? 1u : 0u, &total, S.scan);
-    if (kp) {
-      const uint32_t pos = (uint32_t)(base + ex);
-      const uint32_t s = (uint32_t)(k >> P.b);
-      P.col[pos] = (uint32_t)k & bmask;
-      P.oval[pos] = vin[i];
-      // first kept entry of row s: nothing before it in the sorted order
-      // shares its row (a duplicate of the same key shares it and is not kept)
-      if (i == 0 || (kin[i - 1] >> P.b) != (u64)s) P.ro[s] = pos;
-    }
-    base += total;
-    __syncthreads();
-  }
-  if (gtid == 0) {
-    P.ro[P.n] = (uint32_t)m;
-    *P.m_out = m;
-  }
-  if (!grid_sync(P.bar)) return;
-
-  // ---- empty rows take the offset of the next non-empty row: backward
-  // minimum over ro (ro[n] = m is always set)
-  const uint64_t nr = (uint64_t)P.n + 1;
-  const uint64_t rper = (nr + G - 1) / G;
-  const uint64_t rlo = min(nr, (uint64_t)c * rper), rhi = min(nr, rlo + rper);
+__global__ void __launch_bounds__(kKeepThreads) row_min_kernel(const uint32_t* __restrict__ ro, uint64_t rows,
+                                                               uint32_t* __restrict__ tile_min) {
+  __shared__ uint32_t s_min[32];
   uint32_t mn = 0xffffffffu;
-  for (uint64_t v = rlo + t; v < rhi; v += blockDim.x) mn = min(mn, P.ro[v]);
-  mn = block_suffix_min(mn, S);  // thread 0 holds the range's minimum
-  if (t == 0) P.csum[c] = mn;
-  if (!grid_sync(P.bar)) return;
+#pragma unroll
+  for (uint32_t r = 0; r < kKeepItems; r++) {
+    const uint64_t v = (uint64_t)blockIdx.x * kKeepTile + r * kKeepThreads + threadIdx.x;
+    if (v < rows) mn = min(mn, ro[v]);
+  }
+  mn = block_suffix_min(mn, s_min);
+  if (threadIdx.x == 0) tile_min[blockIdx.x] = mn;
+}
+
+// One block: tile_min[t] = minimum over the tiles after t.
+__global__ void __launch_bounds__(1024) row_carry_kernel(uint32_t* __restrict__ tile_min, uint32_t tiles) {
+  __shared__ uint32_t s_min[32], s_all;
   uint32_t carry = 0xffffffffu;
-  for (uint32_t cc = c + 1; cc < G; cc++) carry = min(carry, (uint32_t)ld_cg(P.csum + cc));
-  if (rhi > rlo) {
-    for (uint64_t e0 = rhi; e0 > rlo;) {
-      const uint64_t b0 = e0 - rlo > blockDim.x ? e0 - blockDim.x : rlo;
-      const uint64_t v = b0 + t;
-      const uint32_t x = v < e0 ? P.ro[v] : 0xffffffffu;
-      const uint32_t y = min(block_suffix_min(x, S), carry);
-      if (v < e0) P.ro[v] = y;
-      // the chunk's minimum (thread 0's suffix) carries to the chunk before
-      if (t == 0) S.scan[0] = y;
-      __syncthreads();
-      carry = S.scan[0];
-      __syncthreads();
-      e0 = b0;
-    }
+  for (uint32_t end = tiles; end;) {
+    const uint32_t beg = end > blockDim.x ? end - blockDim.x : 0u, t = beg + threadIdx.x;
+    const uint32_t x = t < end ? tile_min[t] : 0xffffffffu;
+    // suffix minimum of the tiles after t: shift by one
+    const uint32_t later = t + 1 < end ? tile_min[t + 1] : 0xffffffffu;
+    const uint32_t y = min(block_suffix_min(later, s_min), carry);
+    if (threadIdx.x == 0) s_all = min(min(x, y), carry);
+    __syncthreads();
+    if (t < end) tile_min[t] = y;
+    carry = s_all;
+    __syncthreads();
+    end = beg;
   }
 }
 
+__global__ void __launch_bounds__(kKeepThreads) row_fill_kernel(uint32_t* __restrict__ ro, uint64_t rows,
+                                                                const uint32_t* __restrict__ tile_later) {
+  __shared__ uint32_t s_min[32], s_all;
+  uint32_t carry = tile_later[blockIdx.x];
+  for (uint32_t r = kKeepItems; r--;) {
+    const uint64_t v = (uint64_t)blockIdx.x * kKeepTile + r * kKeepThreads + threadIdx.x;
+    const uint32_t x = v < rows ? ro[v] : 0xffffffffu;
+    const uint32_t y = min(block_suffix_min(x, s_min), carry);
+    if (v < rows && x != y) ro[v] = y;
+    if (threadIdx.x == 0) s_all = y;
+    __syncthreads();
+    carry = s_all;
+    __syncthreads();
+  }
+}
 
 // ---- weight-sorted adjacency (delta-stepping SSSP) ---------------------------
 //
 // Every row of the forward CSR sorted by weight, on the device: the pairs
 // (row << 32 | weight bits, column) of all edges, filled in row order, are
-// radix-sorted on the weight digits and then the row digits (stable, so equal
-// weights keep their column order); weights are non-negative float32 or
-// uint32, whose bit patterns order like the values.  The same pass checks
-// whether the weighted adjacency is symmetric (each row strictly increasing
-// in column, every edge's reverse present with the same weight), which the
-// pull phases of delta-stepping need.
+// radix-sorted (stable, so equal weights keep their column order); weights
+// are non-negative float32 or uint32, whose bit patterns order like the
+// values.  The fill also checks whether the weighted adjacency is symmetric
+// (each row strictly increasing in column, every edge's reverse present with
+// the same weight), which the pull phases of delta-stepping need.
 constexpr uint32_t kWsBig = 256;  // rows at least this long are filled by a whole warp
 
 struct WsortParams {
@@ -279,45 +197,35 @@ struct WsortParams {
   const uint32_t* col;
   const uint32_t* val;
   uint32_t n;
-  uint64_t m;
-  uint32_t passes;  // 4 weight digits + the row digits
   u64* k0;
-  u64* k1;
   uint32_t* v0;
-  uint32_t* v1;
-  uint32_t* hist;       // 256 * gridDim.x
   uint32_t* big;        // rows of at least kWsBig edges (n entries)
   uint32_t* big_count;
   uint32_t* asym;       // set when the adjacency is not symmetric with sorted rows
-  uint32_t* wval;       // out: sorted weights (m)
-  GridBarrier* bar;
 };
 
 // Edge i of row v: its sort pair, and whether it breaks symmetry.
-__device__ __forceinline__ bool ws_edge(const WsortParams& P, uint32_t v, uint64_t i, uint64_t e) {
+__device__ __forceinline__ bool ws_edge(const WsortParams& P, uint32_t v, uint32_t i, uint32_t e) {
   const uint32_t u = P.col[i], w = P.val[i];
   P.k0[i] = ((u64)v << 32) | w;
   P.v0[i] = u;
   if (i + 1 < e && u >= P.col[i + 1]) return true;
   uint32_t lo = P.ro[u], hi = P.ro[u + 1];  // v in row u (sorted): lower bound
+  const uint32_t end = hi;
   while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
+    const uint32_t mid = lo + ((hi - lo) >> 1);
     if (P.col[mid] < v)
       lo = mid + 1;
     else
       hi = mid;
   }
-  return lo == P.ro[u + 1] || P.col[lo] != v || P.val[lo] != w;
+  return lo == end || P.col[lo] != v || P.val[lo] != w;
 }
 
-__global__ void __launch_bounds__(kThreads, 2) wsort_kernel(WsortParams P) {
-  __shared__ Shared S;
-  const uint32_t G = gridDim.x, c = blockIdx.x, lane = threadIdx.x & 31;
-  const uint64_t nth = (uint64_t)G * blockDim.x;
-  const uint64_t gtid = (uint64_t)c * blockDim.x + threadIdx.x;
+// Short rows, one thread each; long rows are listed for whole warps.
+__global__ void __launch_bounds__(256) ws_fill_kernel(WsortParams P) {
   bool bad = false;
-  // ---- fill: short rows one thread each, long rows listed for whole warps
-  for (uint64_t v = gtid; v < P.n; v += nth) {
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < P.n; v += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t b = P.ro[v], e = P.ro[v + 1];
     if (e - b >= kWsBig) {
       P.big[atomicAdd(P.big_count, 1u)] = (uint32_t)v;
@@ -325,25 +233,24 @@ __global__ void __launch_bounds__(kThreads, 2) wsort_kernel(WsortParams P) {
     }
     for (uint32_t i = b; i < e; i++) bad |= ws_edge(P, (uint32_t)v, i, e);
   }
-  if (!grid_sync(P.bar)) return;
-  const uint32_t nbig = ld_cg(P.big_count);
-  for (uint64_t j = gtid >> 5; j < nbig; j += nth >> 5) {
-    const uint32_t v = ld_cg(P.big + j);
+  if (bad) *P.asym = 1u;
+}
+
+__global__ void __launch_bounds__(256) ws_fill_big_kernel(WsortParams P) {
+  const uint32_t nbig = *P.big_count, lane = threadIdx.x & 31u;
+  bool bad = false;
+  for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < nbig; j += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t v = P.big[j];
     const uint32_t b = P.ro[v], e = P.ro[v + 1];
-    for (uint32_t i = b + lane; i < e; i += 32) bad |= ws_edge(P, v, i, e);
+    for (uint64_t i = (uint64_t)b + lane; i < e; i += 32) bad |= ws_edge(P, v, (uint32_t)i, e);
   }
-  if (__any_sync(kFullMask, bad) && lane == 0) atomicOr(P.asym, 1u);
-  if (!grid_sync(P.bar)) return;
-  // ---- sort: weight digits (bits 0-31), then row digits
-  const uint64_t per = (P.m + G - 1) / G;
-  const uint64_t lo = min(P.m, (uint64_t)c * per), hi = min(P.m, lo + per);
-  u64* kin = P.k0;
-  u64* kout = P.k1;
-  uint32_t* vin = P.v0;
-  uint32_t* vout = P.v1;
-  if (!radix_sort_pairs(S, P.bar, P.hist, kin, kout, vin, vout, lo, hi, 0, P.passes)) return;
-  // ---- the sorted weights (the sorted columns stay in vin)
-  for (uint64_t i = gtid; i < P.m; i += nth) P.wval[i] = (uint32_t)kin[i];
+  if (bad) *P.asym = 1u;
+}
+
+__global__ void __launch_bounds__(256) low_words_kernel(const u64* __restrict__ key, uint64_t m,
+                                                        uint32_t* __restrict__ out) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
+    out[i] = (uint32_t)key[i];
 }
 
 }  // namespace gb
@@ -354,72 +261,75 @@ uint32_t bit_length(uint32_t x) { return x ? 32u - (uint32_t)__builtin_clz(x) : 
 
 }  // namespace
 
+// Device arrays of 256-byte alignment cut from one allocation: creating and
+// freeing one costs about 0.6 ms whatever its size, which ten scratch arrays
+// made more than the sort itself.
+struct Carve {
+  uint64_t bytes = 0;
+  char* base = nullptr;
+  uint64_t reserve(uint64_t size) {
+    const uint64_t at = bytes;
+    bytes += (size + 255) / 256 * 256;
+    return at;
+  }
+  template <typename T>
+  T* at(uint64_t offset) const {
+    return reinterpret_cast<T*>(base + offset);
+  }
+};
+
 // Builds g->wcol / g->wval (rows of the forward CSR sorted by weight) and
-// g->wsym once per graph, on the device (wsort_kernel).
+// g->wsym once per graph, on the device.
 sg_status graph_weight_sorted(sg_graph g) {
+  using rsort::u64;
   std::lock_guard<std::mutex> lk(g->wsort_mu);
   if (g->wcol) return SG_OK;
   SG_REQUIRE(g->fwd.val && g->value_type != SG_WEIGHT_NONE, SG_ERR_INVALID, "the graph has no weights");
   const uint32_t n = g->n;
-  const uint64_t m = g->m;
+  const uint64_t m = g->m, ma = m ? m : 1;
   cudaStream_t st = g->stream;
-  gb::WsortParams P = {};
-  P.ro = g->fwd.ro;
-  P.col = g->fwd.col;
-  P.val = reinterpret_cast<const uint32_t*>(g->fwd.val);
-  P.n = n;
-  P.m = m;
-  P.passes = 4 + (bit_length(n - 1) + 7) / 8;
-  const uint64_t grid = 2ull * device_props().sm_count;
-  const uint64_t ma = m ? m : 1;
-  uint32_t* wv = nullptr;
-  uint32_t* flags = nullptr;  // big_count, asym
+  const uint32_t bits = 32 + bit_length(n - 1), passes = (bits + 7) / 8;
+  Carve c;
+  const uint64_t k0 = c.reserve(8 * ma), k1 = c.reserve(8 * ma), v = c.reserve(4 * ma), big = c.reserve(4ull * n),
+                 words = c.reserve(4 * 3), scratch = c.reserve(4 * rsort::scratch_words(m));
+  uint32_t *wc = nullptr, *wv = nullptr;
   sg_status s = SG_OK;
   do {
-    if ((s = dev_alloc(&P.k0, ma)) || (s = dev_alloc(&P.k1, ma)) || (s = dev_alloc(&P.v0, ma)) ||
-        (s = dev_alloc(&P.v1, ma)) || (s = dev_alloc(&P.hist, 256 * grid)) || (s = dev_alloc(&P.big, (uint64_t)n)) ||
-        (s = dev_alloc(&flags, 2)) || (s = dev_alloc(&P.bar, 1)) || (s = dev_alloc(&wv, ma)))
-      break;
-    P.big_count = flags;
-    P.asym = flags + 1;
-    P.wval = wv;
-    cudaError_t e = cudaMemsetAsync(P.bar, 0, sizeof(*P.bar), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), st);
-    if (e != cudaSuccess) {
-      s = cuda_fail(e, "memset", __FILE__, __LINE__);
-      break;
+    if ((s = dev_alloc(&c.base, c.bytes)) || (s = dev_alloc(&wc, ma)) || (s = dev_alloc(&wv, ma))) break;
+    u64* k[2] = {c.at<u64>(k0), c.at<u64>(k1)};
+    uint32_t* vals[2] = {c.at<uint32_t>(v), c.at<uint32_t>(v)};
+    vals[passes & 1] = wc;  // the sorted columns stay where the last pass puts them
+    uint32_t* flags = c.at<uint32_t>(words);  // long rows, asymmetric, m
+    const gb::WsortParams P{g->fwd.ro, g->fwd.col, reinterpret_cast<const uint32_t*>(g->fwd.val),
+                            n,         k[0],       vals[0], c.at<uint32_t>(big), flags, flags + 1};
+    const uint32_t init[3] = {0, 0, (uint32_t)m};
+    cudaError_t e = cudaMemcpyAsync(flags, init, sizeof(init), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && m) {
+      gb::ws_fill_kernel<<<grid_for(n, 256, 8), 256, 0, st>>>(P);
+      gb::ws_fill_big_kernel<<<device_props().sm_count * 8, 256, 0, st>>>(P);
+      count_launch(2);
+      uint32_t done, *left;
+      const rsort::ArraySource src{k[0], vals[0], flags + 2};
+      if ((s = rsort::sort_pairs(src, m, bits, k, vals, c.at<uint32_t>(scratch), st, &done, &left)) != SG_OK) break;
+      gb::low_words_kernel<<<grid_for(m, 256, 8), 256, 0, st>>>(k[passes & 1], m, wv);
+      e = cudaGetLastError();
+      count_launch();
     }
-    if ((s = eng::launch_persistent(gb::wsort_kernel, P, 2, st)) != SG_OK) break;
     uint32_t hf[2] = {0, 0};
-    sygraph::detail::GridBarrier hb;
-    e = cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, P.bar, sizeof(hb), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
       s = cuda_fail(e, "weight sort", __FILE__, __LINE__);
       break;
     }
-    if (hb.error) {
-      s = fail(SG_ERR_TIMEOUT, "weight sort: a grid barrier wait ran out");
-      break;
-    }
-    // after an even number of passes the sorted columns are in v0, else v1
-    uint32_t*& sorted_col = P.passes % 2 == 0 ? P.v0 : P.v1;
-    g->wcol = sorted_col;
-    sorted_col = nullptr;
+    g->wcol = wc;
     g->wval = wv;
-    wv = nullptr;
+    wc = wv = nullptr;
     g->wsym = hf[1] == 0;
     g->bytes += 8ull * m;
   } while (0);
-  dev_free(P.k0);
-  dev_free(P.k1);
-  dev_free(P.v0);
-  dev_free(P.v1);
-  dev_free(P.hist);
-  dev_free(P.big);
-  dev_free(flags);
-  dev_free(P.bar);
+  dev_free(c.base);
+  dev_free(wc);
   dev_free(wv);
   return s;
 }
@@ -427,100 +337,80 @@ sg_status graph_weight_sorted(sg_graph g) {
 namespace {
 
 // One direction (forward, or with src / dst swapped the inverse) of a build;
-// out gets device arrays ro (n+1), col and val (m each).
+// out gets device arrays ro (n+1), col and val (m each) in one allocation.
 sg_status build_direction(const uint32_t* dsrc, const uint32_t* ddst, const uint32_t* dval, uint64_t count,
                           uint32_t n, uint32_t one, int symmetrize, int dedupe, int drop_self_loops,
                           cudaStream_t stream, GraphDir* out, uint64_t* m_out) {
-  const uint64_t E = symmetrize ? 2 * count : count;
-  gb::BuildParams P = {};
-  P.src = dsrc;
-  P.dst = ddst;
-  P.val = dval;
-  P.count = count;
-  P.n = n;
-  P.b = bit_length(n);
-  P.one = one;
-  P.symmetrize = symmetrize;
-  P.dedupe = dedupe;
-  P.drop_self_loops = drop_self_loops;
-  P.entries = E;
-  P.passes = (2 * P.b + 7) / 8;
-  const uint64_t grid = 2ull * device_props().sm_count;  // at least the launch's grid
-  const uint64_t Ea = E ? E : 1;
+  using rsort::u64;
+  const uint64_t E = symmetrize ? 2 * count : count, Ea = E ? E : 1;  // below 2^32
+  const uint32_t b = bit_length(n - 1);
+  const uint32_t tiles = (uint32_t)((Ea - 1) / gb::kKeepTile + 1);
+  const uint64_t rows = (uint64_t)n + 1;
+  const uint32_t row_tiles = (uint32_t)((rows - 1) / gb::kKeepTile + 1);
+  Carve c;
+  const uint64_t k0 = c.reserve(8 * Ea), k1 = c.reserve(8 * Ea), v0 = c.reserve(4 * Ea), v1 = c.reserve(4 * Ea),
+                 scratch = c.reserve(4 * rsort::scratch_words(E)), tile_kept = c.reserve(4ull * tiles),
+                 tile_min = c.reserve(4ull * row_tiles), words = c.reserve(8);
+  void* block = nullptr;
   sg_status s = SG_OK;
-  uint32_t* ro = nullptr;
-  uint32_t* col = nullptr;
-  uint32_t* val = nullptr;
   do {
-    if ((s = dev_alloc(&P.k0, Ea)) || (s = dev_alloc(&P.k1, Ea)) || (s = dev_alloc(&P.v0, Ea)) ||
-        (s = dev_alloc(&P.v1, Ea)) || (s = dev_alloc(&P.hist, 256 * grid)) || (s = dev_alloc(&P.csum, grid)) ||
-        (s = dev_alloc(&ro, (uint64_t)n + 1)) || (s = dev_alloc(&P.m_out, 1)) || (s = dev_alloc(&P.bad, 1)) ||
-        (s = dev_alloc(&P.bar, 1)))
-      break;
-    P.ro = ro;
-    // compacted columns / row ids / values go to the sort buffers that the
-    // last pass leaves free (the pass count decides which ones)
-    const bool even = P.passes % 2 == 0;
-    P.col = reinterpret_cast<uint32_t*>(even ? P.k1 : P.k0);
-    P.oval = even ? P.v1 : P.v0;
-    cudaError_t e = cudaMemsetAsync(P.bar, 0, sizeof(*P.bar), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(P.bad, 0, sizeof(uint32_t), stream);
+    if ((s = dev_alloc(&c.base, c.bytes))) break;
+    uint32_t* flags = c.at<uint32_t>(words);  // edges kept, an endpoint was out of range
+    cudaError_t e = cudaMemsetAsync(flags, 0, 8, stream);
     if (e != cudaSuccess) {
       s = cuda_fail(e, "memset", __FILE__, __LINE__);
       break;
     }
-    if ((s = eng::launch_persistent(gb::build_kernel, P, 2, stream)) != SG_OK) break;
-    uint64_t m = 0;
-    uint32_t bad = 0;
-    sygraph::detail::GridBarrier hb;
-    e = cudaMemcpyAsync(&m, P.m_out, sizeof(m), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, P.bad, sizeof(bad), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, P.bar, sizeof(hb), cudaMemcpyDeviceToHost, stream);
+    const gb::EdgeSource src{dsrc, ddst, dval, (uint32_t)E, n, b, one, symmetrize, drop_self_loops, flags + 1};
+    u64* k[2] = {c.at<u64>(k0), c.at<u64>(k1)};
+    uint32_t* v[2] = {c.at<uint32_t>(v0), c.at<uint32_t>(v1)};
+    uint32_t passes, *left;
+    if ((s = rsort::sort_pairs(src, E, 2 * b, k, v, c.at<uint32_t>(scratch), stream, &passes, &left)) != SG_OK) break;
+    const u64* key = k[passes & 1];
+    uint32_t* kept = c.at<uint32_t>(tile_kept);
+    gb::keep_count_kernel<<<tiles, gb::kKeepThreads, 0, stream>>>(key, left, dedupe, kept);
+    rsort::scan_kernel<<<1, rsort::kSortThreads, 0, stream>>>(tiles, kept, flags);
+    count_launch(2);
+    uint32_t hf[2];
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) {
       s = cuda_fail(e, "graph build", __FILE__, __LINE__);
       break;
     }
-    if (hb.error) {
-      s = fail(SG_ERR_TIMEOUT, "graph build: a grid barrier wait ran out");
-      break;
-    }
-    if (bad) {
+    if (hf[1]) {
       s = fail(SG_ERR_INVALID, "edge endpoint out of range");
       break;
     }
-    if (m >= (1ull << 32)) {
-      s = fail(SG_ERR_INVALID, "edge count must fit uint32 offsets");
+    const uint64_t m = hf[0], ma = m ? m : 1;
+    Carve o;
+    const uint64_t ro = o.reserve(4 * rows), col = o.reserve(4 * ma), val = o.reserve(4 * ma);
+    if ((s = dev_alloc(&o.base, o.bytes))) break;
+    block = o.base;
+    e = cudaMemsetAsync(o.at<uint32_t>(ro), 0xff, 4 * rows, stream);
+    gb::keep_write_kernel<<<tiles, gb::kKeepThreads, 0, stream>>>(key, v[passes & 1], left, dedupe, b, kept, flags, n,
+                                                                  o.at<uint32_t>(ro), o.at<uint32_t>(col),
+                                                                  o.at<uint32_t>(val));
+    gb::row_min_kernel<<<row_tiles, gb::kKeepThreads, 0, stream>>>(o.at<uint32_t>(ro), rows, c.at<uint32_t>(tile_min));
+    gb::row_carry_kernel<<<1, 1024, 0, stream>>>(c.at<uint32_t>(tile_min), row_tiles);
+    gb::row_fill_kernel<<<row_tiles, gb::kKeepThreads, 0, stream>>>(o.at<uint32_t>(ro), rows, c.at<uint32_t>(tile_min));
+    count_launch(4);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) {
+      s = cuda_fail(e, "graph build", __FILE__, __LINE__);
       break;
     }
-    if ((s = dev_alloc(&col, m ? m : 1)) || (s = dev_alloc(&val, m ? m : 1))) break;
-    if (m) {
-      e = cudaMemcpyAsync(col, P.col, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, stream);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(val, P.oval, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-      if (e != cudaSuccess) {
-        s = cuda_fail(e, "graph build copy", __FILE__, __LINE__);
-        break;
-      }
-    }
-    out->ro = ro;
-    out->col = col;
-    out->val = val;
+    out->ro = o.at<uint32_t>(ro);
+    out->col = o.at<uint32_t>(col);
+    out->val = o.at<uint32_t>(val);
+    out->block = block;
     *m_out = m;
-    ro = col = val = nullptr;
+    block = nullptr;
   } while (0);
-  dev_free(P.k0);
-  dev_free(P.k1);
-  dev_free(P.v0);
-  dev_free(P.v1);
-  dev_free(P.hist);
-  dev_free(P.csum);
-  dev_free(P.m_out);
-  dev_free(P.bad);
-  dev_free(P.bar);
-  dev_free(ro);
-  dev_free(col);
-  dev_free(val);
+  dev_free(c.base);
+  if (block) cudaFree(block);
   return s;
 }
 

@@ -72,18 +72,22 @@ __global__ void barrier_check_kernel(sygraph::detail::GridBarrier* bar, uint32_t
 
 using namespace sgb;
 
+static void release_dir(GraphDir& d) {
+  if (d.block) {
+    cudaFree(d.block);
+    return;
+  }
+  dev_free(d.ro);
+  dev_free(d.col);
+  if (d.val) cudaFree(d.val);
+}
+
 void sgb::release_graph(sg_graph g) {
   if (!g) return;
   dev_free(g->wcol);
   if (g->wval) cudaFree(g->wval);
-  if (g->owns_inverse) {
-    dev_free(g->inv.ro);
-    dev_free(g->inv.col);
-    if (g->inv.val) cudaFree(g->inv.val);
-  }
-  dev_free(g->fwd.ro);
-  dev_free(g->fwd.col);
-  if (g->fwd.val) cudaFree(g->fwd.val);
+  if (g->owns_inverse) release_dir(g->inv);
+  release_dir(g->fwd);
   delete g;
 }
 

@@ -113,6 +113,7 @@ struct GraphDir {
   uint32_t* ro = nullptr;
   uint32_t* col = nullptr;
   void* val = nullptr;
+  void* block = nullptr;  // the one allocation behind all three, where they share one
 };
 
 }  // namespace sgb

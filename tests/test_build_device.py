@@ -98,3 +98,18 @@ def test_rmat_edge_list_device_pointers_and_bfs(sg, oracle, rmat):
     b.init(src0)
     b.run(sg.algorithms.bfs_direction.hybrid, 15.0, 24.0)
     assert np.array_equal(b.getDistances(), oracle.bfs_levels(g, src0))
+
+
+@pytest.mark.parametrize("k", [1, 1536, 3071, 3072, 3073, 4096, 4097, 3 * 3072, 70_001])
+@pytest.mark.parametrize("n", [3, 4095, 4096, 4097, 20_000])
+def test_tile_edges(sg, k, n):
+    """Entries around the sort's (3072) and the compaction's (4096) tiles, rows
+    around the offset scan's (4096); few vertices make long runs of equal
+    digits and keys, many make empty rows."""
+    rng = np.random.default_rng(k * 7 + n)
+    s = rng.integers(0, n, k).astype(np.uint32)
+    d = rng.integers(0, max(1, n // 3), k).astype(np.uint32)
+    w = rng.integers(1, 1 << 20, k).astype(np.uint32)
+    for sym, dd, dsl in ((0, 0, 0), (0, 1, 1), (1, 1, 1)):
+        G = sg.graph.build.fromCOO(n, s, d, w, symmetrize=bool(sym), dedupe=bool(dd), drop_self_loops=bool(dsl))
+        _same(sg, G, _host(sg, n, s, d, w, sym, dd, dsl), directed=not sym)
