@@ -385,7 +385,8 @@ sg_status build_direction(const uint32_t* dsrc, const uint32_t* ddst, const uint
     }
     const uint64_t m = hf[0], ma = m ? m : 1;
     Carve o;
-    const uint64_t ro = o.reserve(4 * rows), col = o.reserve(4 * ma), val = o.reserve(4 * ma);
+    const uint64_t ro = o.reserve(4 * rows), col = o.reserve(4 * ma), val = o.reserve(4 * ma), units = o.reserve(4),
+                   unit = o.reserve(sizeof(uint2) * hub_units_capacity(m));
     if ((s = dev_alloc(&o.base, o.bytes))) break;
     block = o.base;
     e = cudaMemsetAsync(o.at<uint32_t>(ro), 0xff, 4 * rows, stream);
@@ -396,16 +397,16 @@ sg_status build_direction(const uint32_t* dsrc, const uint32_t* ddst, const uint
     gb::row_carry_kernel<<<1, 1024, 0, stream>>>(c.at<uint32_t>(tile_min), row_tiles);
     gb::row_fill_kernel<<<row_tiles, gb::kKeepThreads, 0, stream>>>(o.at<uint32_t>(ro), rows, c.at<uint32_t>(tile_min));
     count_launch(4);
+    GraphDir d{o.at<uint32_t>(ro), o.at<uint32_t>(col), o.at<uint32_t>(val), block, o.at<uint32_t>(units),
+               o.at<uint2>(unit)};
     if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess && (s = build_hub_units(d, n, stream)) != SG_OK) break;
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) {
       s = cuda_fail(e, "graph build", __FILE__, __LINE__);
       break;
     }
-    out->ro = o.at<uint32_t>(ro);
-    out->col = o.at<uint32_t>(col);
-    out->val = o.at<uint32_t>(val);
-    out->block = block;
+    *out = d;
     *m_out = m;
     block = nullptr;
   } while (0);
@@ -472,7 +473,7 @@ sg_status sg_graph_create_coo(const uint32_t* src, const uint32_t* dst, const vo
   s = build_direction(dsrc, ddst, dval, count, n, one, symmetrize, dedupe, drop_self_loops, st, &g->fwd, &m);
   if (s == SG_OK) {
     g->m = m;
-    g->bytes = sizeof(uint32_t) * ((uint64_t)n + 1 + 2 * m);
+    g->bytes = sizeof(uint32_t) * ((uint64_t)n + 1 + 2 * m) + sizeof(uint2) * hub_units_capacity(m);
     if (symmetrize) {
       g->inv = g->fwd;
       g->owns_inverse = false;

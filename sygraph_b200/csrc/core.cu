@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "sygraph/detail/advance_kernels.cuh"
 #include "sygraph/detail/primitives.cuh"
 
 namespace sgb {
@@ -80,6 +81,40 @@ static void release_dir(GraphDir& d) {
   dev_free(d.ro);
   dev_free(d.col);
   if (d.val) cudaFree(d.val);
+  dev_free(d.n_hub_units);
+}
+
+uint64_t sgb::hub_units_capacity(uint64_t m) {
+  using namespace sygraph::detail;
+  return m / kHubUnit + m / kHubDegree + 1;
+}
+
+// One thread per row; the order of the units does not matter.
+static __global__ void __launch_bounds__(256) hub_units_kernel(const uint32_t* __restrict__ ro, uint32_t n,
+                                                               uint2* __restrict__ units, uint32_t* count) {
+  using namespace sygraph::detail;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t b = ro[v], d = ro[v + 1] - b;
+    if (d < kHubDegree) continue;
+    const uint32_t k = (d - 1) / kHubUnit + 1;
+    const uint32_t at = atomicAdd(count, k);
+    for (uint32_t j = 0; j < k; j++) units[at + j] = make_uint2((uint32_t)v, b + j * kHubUnit);
+  }
+}
+
+sg_status sgb::build_hub_units(GraphDir& d, uint32_t n, cudaStream_t stream) {
+  SG_CUDA(cudaMemsetAsync(d.n_hub_units, 0, sizeof(uint32_t), stream));
+  if (!n) return SG_OK;
+  hub_units_kernel<<<grid_for(n, 256, 8), 256, 0, stream>>>(d.ro, n, d.hub_units, d.n_hub_units);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
+}
+
+// The same with an allocation of its own: the count in the first 256 bytes.
+static sg_status alloc_hub_units(GraphDir& d, uint32_t n, uint64_t m, cudaStream_t stream) {
+  SG_TRY(dev_alloc(&d.n_hub_units, 64 + 2 * hub_units_capacity(m)));
+  d.hub_units = reinterpret_cast<uint2*>(d.n_hub_units + 64);
+  return build_hub_units(d, n, stream);
 }
 
 void sgb::release_graph(sg_graph g) {
@@ -308,9 +343,10 @@ static sg_status build_inverse(sg_graph g, const uint32_t* h_ro, const uint32_t*
     g->inv.val = d;
     SG_CUDA(cudaMemcpyAsync(d, ival.data(), sizeof(uint32_t) * m, cudaMemcpyHostToDevice, g->stream));
   }
-  SG_CUDA(cudaStreamSynchronize(g->stream));
   g->owns_inverse = true;
-  g->bytes += sizeof(uint32_t) * ((uint64_t)n + 1 + m + (hv ? m : 0));
+  SG_TRY(alloc_hub_units(g->inv, n, m, g->stream));
+  SG_CUDA(cudaStreamSynchronize(g->stream));
+  g->bytes += sizeof(uint32_t) * ((uint64_t)n + 1 + m + (hv ? m : 0)) + sizeof(uint2) * hub_units_capacity(m);
   return SG_OK;
 }
 
@@ -365,7 +401,8 @@ sg_status sg_graph_create_csr(const uint32_t* host_row_offsets, const uint32_t* 
       s = cuda_fail(e, "graph upload", __FILE__, __LINE__);
       break;
     }
-    g->bytes = sizeof(uint32_t) * ((uint64_t)n + 1 + 2 * m);
+    if ((s = alloc_hub_units(g->fwd, n, m, g->stream)) != SG_OK) break;
+    g->bytes = sizeof(uint32_t) * ((uint64_t)n + 1 + 2 * m) + sizeof(uint2) * hub_units_capacity(m);
     if (flags & SG_GRAPH_DIRECTED) {
       if ((s = build_inverse(g, host_row_offsets, host_column_indices, vals)) != SG_OK) break;
     } else {

@@ -28,8 +28,21 @@ MLBDev mlb_dev(const sg_frontier_s* f) {
 
 // One lane per level-0 word.  Push lists words with any bit set; pull
 // (invert) lists words with a clear bit inside [0, num_elems), i.e. words
-// that still hold candidates.  Warp ballot + one atomic per warp.
-__global__ void __launch_bounds__(256) mlb_compact_kernel(MLBDev f, int invert) {
+// that still hold candidates.  Warp ballot + one atomic per warp on the
+// running count, which the last block publishes and clears: one launch
+// instead of a memset and one (an operator loop is a chain of such launches,
+// two to three microseconds each).
+__device__ __forceinline__ bool last_block(uint32_t* done) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+
+__global__ void __launch_bounds__(256) mlb_compact_kernel(MLBDev f, int invert, uint32_t* running, uint32_t* done) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -46,9 +59,24 @@ __global__ void __launch_bounds__(256) mlb_compact_kernel(MLBDev f, int invert) 
         keep = (bits & full) != full;
       }
     }
-    const uint32_t pos = sygraph::detail::warp_append(keep, f.offsets_size);
+    const uint32_t pos = sygraph::detail::warp_append(keep, running);
     if (keep) f.offsets[pos] = (int32_t)w;
   }
+  if (last_block(done) && threadIdx.x == 0) {
+    *f.offsets_size = ld_cg(running);
+    *running = 0;
+    *done = 0;
+  }
+}
+
+// Both levels and the list's size to zero, in one launch.
+__global__ void __launch_bounds__(256) mlb_clear_kernel(MLBDev f) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  uint4* v = reinterpret_cast<uint4*>(f.l0);  // 256-byte aligned
+  for (uint32_t i = t; i < f.words0 / 4; i += nt) v[i] = make_uint4(0, 0, 0, 0);
+  if (t < (f.words0 & 3u)) f.l0[(f.words0 & ~3u) + t] = 0;
+  for (uint32_t i = t; i < f.words1; i += nt) f.l1[i] = 0;
+  if (t == 0) *f.offsets_size = 0;
 }
 
 __global__ void mlb_insert_one(MLBDev f, uint32_t idx) { f.insert(idx); }
@@ -82,34 +110,45 @@ __global__ void __launch_bounds__(256) mlb_bitwise(uint32_t* dst, const uint32_t
   }
 }
 
-// Population count of level 0 and any-non-zero flag.
-__global__ void __launch_bounds__(256) mlb_count(MLBDev f, unsigned long long* out) {
+// Population count of level 0 (its non-zero words when `any`), left by the
+// last block in pinned host memory: no memset before and no copy after.
+__global__ void __launch_bounds__(256) mlb_count(MLBDev f, bool any, unsigned long long* sum, uint32_t* done,
+                                                 volatile unsigned long long* host) {
   __shared__ unsigned long long s_red[32];
   unsigned long long c = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.words0; i += gridDim.x * blockDim.x)
-    c += __popc(ld_cg(f.l0 + i));
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.words0; i += gridDim.x * blockDim.x) {
+    const uint32_t w = ld_cg(f.l0 + i);
+    c += any ? (w != 0) : __popc(w);
+  }
   c = sygraph::detail::block_sum(c, s_red);
-  if (threadIdx.x == 0 && c) atomicAdd(out, c);
+  if (threadIdx.x == 0 && c) atomicAdd(sum, c);
+  if (last_block(done) && threadIdx.x == 0) {
+    *host = ld_cg(sum);
+    *sum = 0;
+    *done = 0;
+  }
 }
 
-__global__ void __launch_bounds__(256) mlb_any(MLBDev f, unsigned long long* out) {
-  bool any = false;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < f.words0 && !any; i += gridDim.x * blockDim.x)
-    any = ld_cg(f.l0 + i) != 0;
-  if (__any_sync(kFullMask, any) && (threadIdx.x & 31) == 0) atomicOr(out, 1ull);
+static sg_status frontier_count(sg_frontier f, bool any, uint64_t* out) {
+  uint32_t* words = reinterpret_cast<uint32_t*>(f->scratch);
+  mlb_count<<<grid_for(f->words0, 1024), 256, 0, f->stream>>>(mlb_dev(f), any, (unsigned long long*)f->scratch,
+                                                             words + 4, (unsigned long long*)f->host_word);
+  SG_CHECK_LAUNCH();
+  SG_CUDA(cudaStreamSynchronize(f->stream));
+  *out = *f->host_word;
+  return SG_OK;
 }
 
 sg_status frontier_compact(sg_frontier f, int invert, cudaStream_t stream) {
-  SG_CUDA(cudaMemsetAsync(f->offsets_size, 0, sizeof(uint32_t), stream));
-  mlb_compact_kernel<<<grid_for(f->words0, 256), 256, 0, stream>>>(mlb_dev(f), invert);
+  uint32_t* words = reinterpret_cast<uint32_t*>(f->scratch);
+  mlb_compact_kernel<<<grid_for(f->words0, 256), 256, 0, stream>>>(mlb_dev(f), invert, words + 2, words + 3);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
 
 sg_status frontier_clear(sg_frontier f, cudaStream_t stream) {
-  SG_CUDA(cudaMemsetAsync(f->level0, 0, sizeof(uint32_t) * f->words0, stream));
-  SG_CUDA(cudaMemsetAsync(f->level1, 0, sizeof(uint32_t) * f->words1, stream));
-  SG_CUDA(cudaMemsetAsync(f->offsets_size, 0, sizeof(uint32_t), stream));
+  mlb_clear_kernel<<<grid_for(f->words0, 1024), 256, 0, stream>>>(mlb_dev(f));
+  SG_CHECK_LAUNCH();
   return SG_OK;
 }
 
@@ -132,11 +171,8 @@ using namespace sgb;
 
 static void frontier_release(sg_frontier f) {
   if (!f) return;
-  dev_free(f->level0);
-  dev_free(f->level1);
-  dev_free(f->offsets);
-  dev_free(f->offsets_size);
-  dev_free(f->scratch);
+  if (f->block) cudaFree(f->block);
+  if (f->host_word) cudaFreeHost(f->host_word);
   delete f;
 }
 
@@ -151,10 +187,22 @@ sg_status sg_frontier_create(uint32_t num_elems, void* stream, sg_frontier* out)
   f->words0 = div_up(num_elems, 32);
   f->words1 = div_up(f->words0, 32);
   f->stream = (cudaStream_t)stream;
-  sg_status s;
-  if ((s = dev_alloc(&f->level0, f->words0)) || (s = dev_alloc(&f->level1, f->words1)) ||
-      (s = dev_alloc(&f->offsets, f->words0)) || (s = dev_alloc(&f->offsets_size, 1)) ||
-      (s = dev_alloc(&f->scratch, 1)) || (s = frontier_clear(f, f->stream))) {
+  // one allocation: level 0, level 1, the word list, its size, the scratch words
+  const uint64_t l0 = ((uint64_t)f->words0 * 4 + 255) / 256 * 256, l1 = ((uint64_t)f->words1 * 4 + 255) / 256 * 256;
+  char* base = nullptr;
+  sg_status s = dev_alloc(&base, 2 * l0 + l1 + 512);
+  f->block = base;
+  if (s == SG_OK) {
+    f->level0 = reinterpret_cast<uint32_t*>(base);
+    f->level1 = reinterpret_cast<uint32_t*>(base + l0);
+    f->offsets = reinterpret_cast<int32_t*>(base + l0 + l1);
+    f->offsets_size = reinterpret_cast<uint32_t*>(base + 2 * l0 + l1);
+    f->scratch = reinterpret_cast<uint64_t*>(base + 2 * l0 + l1 + 256);
+    cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&f->host_word), sizeof(uint64_t));
+    if (e == cudaSuccess) e = cudaMemsetAsync(f->scratch, 0, 256, f->stream);
+    if (e != cudaSuccess) s = cuda_fail(e, "frontier set-up", __FILE__, __LINE__);
+  }
+  if (s != SG_OK || (s = frontier_clear(f, f->stream))) {
     frontier_release(f);
     return s;
   }
@@ -235,24 +283,15 @@ sg_status sg_frontier_insert_list(sg_frontier f, const uint32_t* host_ids, uint6
 
 sg_status sg_frontier_empty(sg_frontier f, int* empty) {
   SG_REQUIRE(f && empty, SG_ERR_INVALID, "NULL argument");
-  SG_CUDA(cudaMemsetAsync(f->scratch, 0, sizeof(uint64_t), f->stream));
-  mlb_any<<<grid_for(f->words0, 256), 256, 0, f->stream>>>(mlb_dev(f), (unsigned long long*)f->scratch);
-  SG_CHECK_LAUNCH();
   uint64_t any = 0;
-  SG_CUDA(cudaMemcpyAsync(&any, f->scratch, sizeof(any), cudaMemcpyDeviceToHost, f->stream));
-  SG_CUDA(cudaStreamSynchronize(f->stream));
+  SG_TRY(frontier_count(f, true, &any));
   *empty = any ? 0 : 1;
   return SG_OK;
 }
 
 sg_status sg_frontier_size(sg_frontier f, uint64_t* size) {
   SG_REQUIRE(f && size, SG_ERR_INVALID, "NULL argument");
-  SG_CUDA(cudaMemsetAsync(f->scratch, 0, sizeof(uint64_t), f->stream));
-  mlb_count<<<grid_for(f->words0, 256), 256, 0, f->stream>>>(mlb_dev(f), (unsigned long long*)f->scratch);
-  SG_CHECK_LAUNCH();
-  SG_CUDA(cudaMemcpyAsync(size, f->scratch, sizeof(uint64_t), cudaMemcpyDeviceToHost, f->stream));
-  SG_CUDA(cudaStreamSynchronize(f->stream));
-  return SG_OK;
+  return frontier_count(f, false, size);
 }
 
 sg_status sg_frontier_merge(sg_frontier f, sg_frontier other) {
@@ -281,6 +320,7 @@ sg_status sg_frontier_swap(sg_frontier a, sg_frontier b) {
   std::swap(a->offsets, b->offsets);
   std::swap(a->offsets_size, b->offsets_size);
   std::swap(a->scratch, b->scratch);
+  std::swap(a->block, b->block);
   return SG_OK;
 }
 

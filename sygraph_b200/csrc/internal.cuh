@@ -113,8 +113,17 @@ struct GraphDir {
   uint32_t* ro = nullptr;
   uint32_t* col = nullptr;
   void* val = nullptr;
-  void* block = nullptr;  // the one allocation behind all three, where they share one
+  void* block = nullptr;  // the one allocation behind all of it, where they share one
+  // long rows in units for the operators' advances (advance_kernels.cuh): the
+  // count, and hub_units(count) as (vertex, first edge)
+  uint32_t* n_hub_units = nullptr;
+  uint2* hub_units = nullptr;
 };
+
+// Bytes of a direction's unit list (at most m / kHubUnit full units and one
+// more for each of at most m / kHubDegree rows), and its build on the device.
+uint64_t hub_units_capacity(uint64_t m);
+sg_status build_hub_units(GraphDir& d, uint32_t n, cudaStream_t stream);
 
 }  // namespace sgb
 
@@ -158,7 +167,12 @@ struct sg_frontier_s {
   uint32_t* level1 = nullptr;
   int32_t* offsets = nullptr;
   uint32_t* offsets_size = nullptr;
-  uint64_t* scratch = nullptr;  // device scalar for reductions
+  // device words, zero between launches: [0] a count's sum, the low and high
+  // half of [1] the compaction's running count and its blocks done, [2] the
+  // count's blocks done; [4] the sum of compute::reduce
+  uint64_t* scratch = nullptr;
+  uint64_t* host_word = nullptr;  // pinned: where the device leaves empty()'s and size()'s answer
+  void* block = nullptr;          // the one device allocation behind all of it
   cudaStream_t stream = nullptr;
   sg_frontier_view view() const {
     sg_frontier_view v;

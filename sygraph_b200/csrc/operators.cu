@@ -160,6 +160,9 @@ sg_status sg_advance(sg_graph g, sg_frontier in, sg_frontier out, int direction,
     SG_TRY(frontier_compact(in, direction != SG_DIR_PUSH, s));
   }
   if (out_view == SG_VIEW_VERTEX) a.out = mlb_dev(out);
+  const GraphDir& dir = direction != SG_DIR_PUSH ? g->inv : g->fwd;
+  a.hub_units = dir.hub_units;
+  a.n_hub_units = dir.n_hub_units;
   const sg_graph_view v = g->view(direction != SG_DIR_PUSH);
   return dispatch(op, x, direction, load_balancer, v, a, advance_grid(expected_size), s);
 }
@@ -225,9 +228,9 @@ sg_status sg_compute_reduce(sg_graph g, sg_frontier f, int fn, const sg_op_args*
   (void)args;
   cudaStream_t s = g->stream;
   SG_TRY(frontier_compact(f, 0, s));
-  SG_CUDA(cudaMemsetAsync(f->scratch, 0, sizeof(uint64_t), s));
+  unsigned long long* acc = (unsigned long long*)f->scratch + 4;  // (the words before it stay zero between launches)
+  SG_CUDA(cudaMemsetAsync(acc, 0, sizeof(uint64_t), s));
   const unsigned grid = grid_for((uint64_t)f->words0 * 32, 256);
-  unsigned long long* acc = (unsigned long long*)f->scratch;
   switch (fn) {
     case SG_RED_VERTEX_ID: compute_reduce_kernel<<<grid, 256, 0, s>>>(mlb_dev(f), g->n, ops::RedVertexId{}, acc); break;
     case SG_RED_DEGREE:

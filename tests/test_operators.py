@@ -242,3 +242,43 @@ def test_compute_reduce_degree_and_segmented_intersection(sg, ops, rmat, oracle)
     ro, col = g.row_offsets, g.column_indices
     want = [len(np.intersect1d(col[ro[x]:ro[x + 1]], col[ro[y]:ro[y + 1]])) for x, y in zip(a, b)]
     assert got.tolist() == want
+
+
+@pytest.mark.parametrize("lb", [2, 3])
+@pytest.mark.parametrize("directed", [False, True])
+def test_advance_long_rows(sg, ops, lb, directed):
+    """Rows around the long-row limit (512 edges) and the unit size (1024):
+    every edge of a candidate is visited exactly once in push and pull_all,
+    at least once where a pull succeeds, from device-built and uploaded graphs."""
+    degs = [1, 31, 32, 511, 512, 513, 1023, 1024, 1025, 2047, 2048, 2049, 5000]
+    n = 6000
+    rng = np.random.default_rng(17)
+    s = np.concatenate([np.full(d, h) for h, d in enumerate(degs)])
+    d = np.concatenate([rng.choice(np.arange(100, n), k, replace=False) for k in degs])
+    g = sg.io.fromCOO(n, s, d, symmetrize=not directed, dedupe=True)
+    graphs = [sg.graph.build.fromCSR(g, sg.Properties(directed=directed)),
+              sg.graph.build.fromCOO(n, s, d, symmetrize=not directed, dedupe=True)]
+    inv = g.invert() if directed else g
+    for G in graphs:
+        for density in (0.02, 0.9):
+            flags = (rng.random(n) < density).astype(np.uint8)
+            flags[:len(degs)] = rng.random(len(degs)) < 0.5
+            for direction in (0, 1, 2):
+                fin, fout = sg.frontier.makeFrontier(G), sg.frontier.makeFrontier(G)
+                fin.insert_list(np.nonzero(flags)[0])
+                assert fin.size() == int(flags.sum()) and not fin.empty()
+                visits = sg.DeviceArray(np.zeros(n, np.uint32))
+                ops.advance.frontier(G, fin, fout, ops.OP_COUNT_VISITS, ops.op_args([visits]), direction, lb)
+                got, c = visits.numpy(), g if direction == 0 else inv
+                ro, col = c.row_offsets, c.column_indices
+                if direction == 0:
+                    want = np.where(flags, c.degrees(), 0)
+                else:
+                    want = np.array([0 if flags[v] else int(flags[col[ro[v]:ro[v + 1]]].sum()) for v in range(n)])
+                if direction == 1:
+                    assert np.array_equal(got > 0, want > 0) and (got <= want).all()
+                else:
+                    assert np.array_equal(got, want)
+                assert np.array_equal(fout.flags(), reference_advance(ro, col, flags, direction))
+                fout.clear()
+                assert fout.empty() and fout.size() == 0
