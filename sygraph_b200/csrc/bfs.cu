@@ -219,6 +219,23 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_kernel(Params P) {
     P.result[3] = visited_vertices;
     P.result[4] = P.m - unexplored;
   }
+  if (blockIdx.x == 0 && P.report.at) {
+    // the step bits, from the log that this block's thread 0 kept
+    __syncthreads();
+    const uint32_t steps = min(level + 1, kMaxLog);
+    for (uint32_t i = threadIdx.x; i < (steps + 31u & ~31u); i += blockDim.x) {
+      const uint32_t w = __ballot_sync(kFullMask, i < steps && ld_cg(&P.log[i].strategy) >= 2u);
+      if ((i & 31u) == 0) {
+        *const_cast<volatile uint32_t*>(P.report.at->pull + (i >> 5)) = w;
+        __threadfence_system();
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {  // (this thread wrote the results)
+      const volatile unsigned long long* r = P.result;
+      report_run(P.report, r[0], r[1], r[2], r[3], r[4]);
+    }
+  }
   {
     // n+1 for every vertex not reached: reached = visited, minus the vertices
     // pre-marked for having no in-edge, plus the source.  Four vertices per
@@ -296,6 +313,8 @@ struct sg_bfs_s {
   sygraph::detail::GridBarrier* bar = nullptr;
   sg_level_record* log = nullptr;
   unsigned long long* result = nullptr;
+  eng::RunReport report;
+  void* block = nullptr;  // the one device allocation behind the arrays above
   int* schedule = nullptr;
   uint32_t schedule_len = 0;
   const sygraph::detail::MlpParams* mlp = nullptr;  // not owned
@@ -328,18 +347,8 @@ static sg_status bfs_materialise(sg_bfs b) {
 
 static void bfs_release(sg_bfs b) {
   if (!b) return;
-  dev_free(b->depth);
-  dev_free(b->visited);
-  dev_free(b->fb);
-  dev_free(b->sm);
-  dev_free(b->no_in);
-  dev_free(b->first_in);
-  dev_free(b->heavy_v);
-  dev_free(b->heavy_s);
-  dev_free(b->cnt);
-  dev_free(b->bar);
-  dev_free(b->log);
-  dev_free(b->result);
+  if (b->block) cudaFree(b->block);
+  b->report.release();
   dev_free(b->schedule);
   dev_free(b->features);
   delete b;
@@ -386,6 +395,7 @@ static sg_status bfs_launch(sg_bfs b, int direction, float alpha, float beta) {
   P.bar = b->bar;
   P.log = b->log;
   P.result = b->result;
+  P.report = b->report.next();
   P.schedule = b->schedule_len ? b->schedule : nullptr;
   P.schedule_len = b->schedule_len;
   if (b->bar_reset) {
@@ -396,31 +406,22 @@ static sg_status bfs_launch(sg_bfs b, int direction, float alpha, float beta) {
 }
 
 static sg_status bfs_collect(sg_bfs b, sg_bfs_details* details) {
-  unsigned long long res[5];
-  sygraph::detail::GridBarrier bar;
-  SG_CUDA(cudaMemcpyAsync(res, b->result, sizeof(res), cudaMemcpyDeviceToHost, b->stream));
-  SG_CUDA(cudaMemcpyAsync(&bar, b->bar, sizeof(bar), cudaMemcpyDeviceToHost, b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
-  if (bar.error) {
+  if (!b->report.finished()) {
     b->bar_reset = true;
     return fail(SG_ERR_TIMEOUT, "BFS engine: a grid barrier wait ran out");
   }
+  const unsigned long long* res = b->report.host->v;
   b->last_iterations = (uint32_t)res[0];
   if (details) {
-    memset(details, 0, sizeof(*details));
     details->iterations = res[0];
     details->push_steps = res[1];
     details->pull_steps = res[2];
     details->visited_vertices = res[3];
     details->visited_edges = res[4];
     const uint32_t nlog = res[0] < SG_MAX_LOGGED_LEVELS ? (uint32_t)res[0] : SG_MAX_LOGGED_LEVELS;
-    // (a std::vector of this C struct trips an internal error of nvcc 12.9's
-    // front end under -std=c++20)
-    std::unique_ptr<sg_level_record[]> recs(new sg_level_record[nlog ? nlog : 1]);
-    if (nlog) {
-      SG_CUDA(cudaMemcpy(recs.get(), b->log, sizeof(sg_level_record) * nlog, cudaMemcpyDeviceToHost));
-      for (uint32_t i = 0; i < nlog; i++) details->step_is_pull[i] = recs[i].strategy >= 2;
-    }
+    memset(details->step_is_pull, 0, SG_MAX_LOGGED_LEVELS);
+    for (uint32_t i = 0; i < nlog; i++) details->step_is_pull[i] = (b->report.host->pull[i >> 5] >> (i & 31)) & 1u;
   }
   return SG_OK;
 }
@@ -440,15 +441,30 @@ sg_status sg_bfs_create(sg_graph g, sg_bfs* out) {
   const uint64_t n = g->n;
   // at most m / kHeavy vertices have degree >= kHeavy
   b->heavy_cap = (uint32_t)std::min<uint64_t>(n, g->m / bfs::kHeavy + 1);
-  sg_status s = SG_OK;
-  if ((s = dev_alloc(&b->depth, n)) || (s = dev_alloc(&b->visited, b->w0)) || (s = dev_alloc(&b->fb, 3ull * b->w0)) ||
-      (s = dev_alloc(&b->sm, 3ull * b->w1)) || (s = dev_alloc(&b->no_in, b->w0)) || (s = dev_alloc(&b->first_in, n)) ||
-      (s = dev_alloc(&b->heavy_v, 2ull * b->heavy_cap)) || (s = dev_alloc(&b->heavy_s, 2ull * b->heavy_cap)) ||
-      (s = dev_alloc(&b->cnt, 3)) || (s = dev_alloc(&b->bar, 1)) || (s = dev_alloc(&b->log, SG_MAX_LOGGED_LEVELS)) ||
-      (s = dev_alloc(&b->result, 8))) {
+  Carve c;
+  const uint64_t depth = c.reserve(4 * n), visited = c.reserve(4ull * b->w0), fb = c.reserve(12ull * b->w0),
+                 sm = c.reserve(12ull * b->w1), no_in = c.reserve(4ull * b->w0), first_in = c.reserve(4 * n),
+                 heavy_v = c.reserve(8ull * b->heavy_cap), heavy_s = c.reserve(8ull * b->heavy_cap),
+                 cnt = c.reserve(3 * sizeof(bfs::LevelCounters)), bar = c.reserve(sizeof(*b->bar)),
+                 log = c.reserve(SG_MAX_LOGGED_LEVELS * sizeof(sg_level_record)), result = c.reserve(8 * 8);
+  sg_status s = dev_alloc(&c.base, c.bytes);
+  b->block = c.base;
+  if (s != SG_OK || (s = b->report.alloc()) != SG_OK) {
     bfs_release(b);
     return s;
   }
+  b->depth = c.at<uint32_t>(depth);
+  b->visited = c.at<uint32_t>(visited);
+  b->fb = c.at<uint32_t>(fb);
+  b->sm = c.at<uint32_t>(sm);
+  b->no_in = c.at<uint32_t>(no_in);
+  b->first_in = c.at<uint32_t>(first_in);
+  b->heavy_v = c.at<uint32_t>(heavy_v);
+  b->heavy_s = c.at<uint32_t>(heavy_s);
+  b->cnt = c.at<bfs::LevelCounters>(cnt);
+  b->bar = c.at<sygraph::detail::GridBarrier>(bar);
+  b->log = c.at<sg_level_record>(log);
+  b->result = c.at<unsigned long long>(result);
   bfs::no_in_edges_kernel<<<grid_for((uint64_t)b->w0 * 32, 256), 256, 0, g->stream>>>(g->inv.ro, g->n, b->w0,
                                                                                        b->no_in);
   bfs::first_in_kernel<<<grid_for(n, 256), 256, 0, g->stream>>>(g->inv.ro, g->inv.col, g->n, b->first_in);
@@ -527,11 +543,10 @@ sg_status sg_bfs_set_schedule(sg_bfs b, const int* host_strategies, uint32_t len
 }  // extern "C"
 
 sg_status sgb::bfs_launch_status(sg_bfs b) {
-  uint32_t err = 0;
-  SG_CUDA(cudaMemcpyAsync(&err, &b->bar->error, sizeof(err), cudaMemcpyDeviceToHost, b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
-  if (err) b->bar_reset = true;
-  return err ? fail(SG_ERR_TIMEOUT, "BFS engine: a grid barrier wait ran out") : SG_OK;
+  if (b->report.finished()) return SG_OK;
+  b->bar_reset = true;
+  return fail(SG_ERR_TIMEOUT, "BFS engine: a grid barrier wait ran out");
 }
 
 extern "C" {

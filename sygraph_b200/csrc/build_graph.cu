@@ -261,23 +261,6 @@ uint32_t bit_length(uint32_t x) { return x ? 32u - (uint32_t)__builtin_clz(x) : 
 
 }  // namespace
 
-// Device arrays of 256-byte alignment cut from one allocation: creating and
-// freeing one costs about 0.6 ms whatever its size, which ten scratch arrays
-// made more than the sort itself.
-struct Carve {
-  uint64_t bytes = 0;
-  char* base = nullptr;
-  uint64_t reserve(uint64_t size) {
-    const uint64_t at = bytes;
-    bytes += (size + 255) / 256 * 256;
-    return at;
-  }
-  template <typename T>
-  T* at(uint64_t offset) const {
-    return reinterpret_cast<T*>(base + offset);
-  }
-};
-
 // Builds g->wcol / g->wval (rows of the forward CSR sorted by weight) and
 // g->wsym once per graph, on the device.
 sg_status graph_weight_sorted(sg_graph g) {

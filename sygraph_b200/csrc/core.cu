@@ -73,6 +73,46 @@ __global__ void barrier_check_kernel(sygraph::detail::GridBarrier* bar, uint32_t
 
 using namespace sgb;
 
+namespace {
+std::mutex g_pinned_mu;
+char* g_pinned_slab = nullptr;  // kept for the process once it exists
+bool g_pinned_used[kPinnedPieces] = {};
+}  // namespace
+
+sg_status sgb::pinned_take(void** piece) {
+  *piece = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    if (!g_pinned_slab && cudaHostAlloc(reinterpret_cast<void**>(&g_pinned_slab), kPinnedPiece * kPinnedPieces,
+                                        cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      g_pinned_slab = nullptr;
+      return fail(SG_ERR_NOMEM, "pinned host memory for results");
+    }
+    for (size_t i = 0; i < kPinnedPieces; i++)
+      if (!g_pinned_used[i]) {
+        g_pinned_used[i] = true;
+        *piece = g_pinned_slab + i * kPinnedPiece;
+        return SG_OK;
+      }
+  }
+  SG_CUDA(cudaHostAlloc(piece, kPinnedPiece, cudaHostAllocPortable));
+  return SG_OK;
+}
+
+void sgb::pinned_give(void* piece) {
+  if (!piece) return;
+  {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    char* p = static_cast<char*>(piece);
+    if (g_pinned_slab && p >= g_pinned_slab && p < g_pinned_slab + kPinnedPiece * kPinnedPieces) {
+      g_pinned_used[(p - g_pinned_slab) / kPinnedPiece] = false;
+      return;
+    }
+  }
+  cudaFreeHost(piece);
+}
+
 static void release_dir(GraphDir& d) {
   if (d.block) {
     cudaFree(d.block);

@@ -277,6 +277,54 @@ __device__ __forceinline__ uint32_t valid_bits(uint32_t wi, uint32_t w0, uint32_
   return (wi == w0 - 1 && rem) ? ((1u << rem) - 1u) : 0xffffffffu;
 }
 
+// What a run leaves in pinned host memory for the host to read when the stream
+// is idle: its totals, and last its number, without which it did not finish
+// (a barrier wait ran out).  Two or three small copies from the device, each
+// about 8 us with its wait, were a third of a small graph's run.
+struct HostReport {
+  unsigned long long v[5];
+  unsigned long long run;
+  uint32_t pull[kMaxLog / 32];  // BFS: bit i % 32 of word i / 32 = step i pulled
+};
+struct ReportRef {
+  HostReport* at = nullptr;  // null: nobody reads one
+  unsigned long long run = 0;
+};
+
+__device__ __forceinline__ void report_run(const ReportRef& r, unsigned long long a, unsigned long long b,
+                                           unsigned long long c, unsigned long long d, unsigned long long e) {
+  if (!r.at) return;
+  volatile unsigned long long* v = r.at->v;
+  v[0] = a;
+  v[1] = b;
+  v[2] = c;
+  v[3] = d;
+  v[4] = e;
+  __threadfence_system();
+  *reinterpret_cast<volatile unsigned long long*>(&r.at->run) = r.run;
+}
+
+// The host's side, one per instance.
+struct RunReport {
+  HostReport* host = nullptr;
+  unsigned long long run = 0;  // the latest launch's number
+  sg_status alloc() {
+    static_assert(sizeof(HostReport) <= kPinnedPiece, "a report is one piece");
+    void* p = nullptr;
+    SG_TRY(pinned_take(&p));
+    host = static_cast<HostReport*>(p);
+    host->run = 0;
+    return SG_OK;
+  }
+  void release() {
+    pinned_give(host);
+    host = nullptr;
+  }
+  ReportRef next() { return ReportRef{host, ++run}; }
+  // once the stream is idle
+  bool finished() const { return *const_cast<volatile unsigned long long*>(&host->run) == run; }
+};
+
 // Cooperative launch with a grid that fills every SM `blocks_per_sm` times,
 // or at most `max_grid` CTAs (a share of the GPU, so that launches on other
 // streams can be resident at the same time).

@@ -172,7 +172,7 @@ using namespace sgb;
 static void frontier_release(sg_frontier f) {
   if (!f) return;
   if (f->block) cudaFree(f->block);
-  if (f->host_word) cudaFreeHost(f->host_word);
+  pinned_give(f->host_word);
   delete f;
 }
 
@@ -198,9 +198,13 @@ sg_status sg_frontier_create(uint32_t num_elems, void* stream, sg_frontier* out)
     f->offsets = reinterpret_cast<int32_t*>(base + l0 + l1);
     f->offsets_size = reinterpret_cast<uint32_t*>(base + 2 * l0 + l1);
     f->scratch = reinterpret_cast<uint64_t*>(base + 2 * l0 + l1 + 256);
-    cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&f->host_word), sizeof(uint64_t));
-    if (e == cudaSuccess) e = cudaMemsetAsync(f->scratch, 0, 256, f->stream);
-    if (e != cudaSuccess) s = cuda_fail(e, "frontier set-up", __FILE__, __LINE__);
+    void* piece = nullptr;
+    s = pinned_take(&piece);
+    f->host_word = static_cast<uint64_t*>(piece);
+    if (s == SG_OK) {
+      cudaError_t e = cudaMemsetAsync(f->scratch, 0, 256, f->stream);
+      if (e != cudaSuccess) s = cuda_fail(e, "frontier set-up", __FILE__, __LINE__);
+    }
   }
   if (s != SG_OK || (s = frontier_clear(f, f->stream))) {
     frontier_release(f);

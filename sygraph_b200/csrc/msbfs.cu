@@ -105,6 +105,7 @@ struct Params {
   uint32_t* depth;   // k * n, source-major, written after the last level
   sg_level_record* log;
   u64* result;       // [iterations, push, pull, reached_edges]
+  ReportRef report;
   const int* schedule;    // optional direction per level: 0 push, 2 pull, -1 the mode decides
   uint32_t schedule_len;
   const sygraph::detail::MlpStaged* mlp_image;  // learned mode: the selector, staged per launch
@@ -693,6 +694,7 @@ __global__ void __launch_bounds__(kThreads, 2) msbfs_kernel(Params P) {
     P.result[1] = n_push;
     P.result[2] = n_pull;
     P.result[3] = reached_total;
+    report_run(P.report, level + 1, n_push, n_pull, reached_total, 0);
   }
 }
 
@@ -731,6 +733,7 @@ struct sg_msbfs_s {
   sygraph::detail::GridBarrier* bar = nullptr;
   sg_level_record* log = nullptr;
   unsigned long long* result = nullptr;
+  eng::RunReport report;
   uint32_t last_k = 0;
   int* schedule = nullptr;  // forced direction per level (device)
   uint32_t schedule_len = 0;
@@ -758,6 +761,7 @@ static void msbfs_release(sg_msbfs h) {
   dev_free(h->bar);
   dev_free(h->log);
   dev_free(h->result);
+  h->report.release();
   dev_free(h->schedule);
   dev_free(h->features);
   delete h;
@@ -788,7 +792,7 @@ sg_status sg_msbfs_create(sg_graph g, uint32_t max_sources, sg_msbfs* out) {
       (s = dev_alloc(&h->heavy_v, 2ull * h->heavy_cap)) || (s = dev_alloc(&h->heavy_s, 2ull * h->heavy_cap)) ||
       (s = dev_alloc(&h->sources, 64)) || (s = dev_alloc(&h->depth, (uint64_t)max_sources * n)) ||
       (s = dev_alloc(&h->cnt, 3)) || (s = dev_alloc(&h->bar, 1)) || (s = dev_alloc(&h->log, SG_MAX_LOGGED_LEVELS)) ||
-      (s = dev_alloc(&h->result, 8))) {
+      (s = dev_alloc(&h->result, 8)) || (s = h->report.alloc())) {
     msbfs_release(h);
     return s;
   }
@@ -884,6 +888,7 @@ sg_status sg_msbfs_run_async(sg_msbfs h, const uint32_t* host_sources, uint32_t 
   P.depth = h->depth;
   P.log = h->log;
   P.result = h->result;
+  P.report = h->report.next();
   P.schedule = h->schedule;
   P.schedule_len = h->schedule_len;
   P.mlp_image = static_cast<const sygraph::detail::MlpStaged*>(h->mlp_image);
@@ -898,12 +903,8 @@ sg_status sg_msbfs_run_async(sg_msbfs h, const uint32_t* host_sources, uint32_t 
 sg_status sg_msbfs_run(sg_msbfs h, const uint32_t* host_sources, uint32_t k, int direction, float alpha, float beta,
                        sg_msbfs_details* details) {
   SG_TRY(sg_msbfs_run_async(h, host_sources, k, direction, alpha, beta));
-  unsigned long long r[4];
-  sygraph::detail::GridBarrier b;
-  SG_CUDA(cudaMemcpyAsync(r, h->result, sizeof(r), cudaMemcpyDeviceToHost, h->stream));
-  SG_CUDA(cudaMemcpyAsync(&b, h->bar, sizeof(b), cudaMemcpyDeviceToHost, h->stream));
-  SG_CUDA(cudaStreamSynchronize(h->stream));
-  if (b.error) return fail(SG_ERR_TIMEOUT, "multi-source BFS: a grid barrier wait ran out");
+  SG_TRY(msbfs_launch_status(h));
+  const unsigned long long* r = h->report.host->v;
   if (details) {
     details->iterations = r[0];
     details->push_steps = r[1];
@@ -916,10 +917,8 @@ sg_status sg_msbfs_run(sg_msbfs h, const uint32_t* host_sources, uint32_t k, int
 }  // extern "C"
 
 sg_status sgb::msbfs_launch_status(sg_msbfs h) {
-  uint32_t err = 0;
-  SG_CUDA(cudaMemcpyAsync(&err, &h->bar->error, sizeof(err), cudaMemcpyDeviceToHost, h->stream));
   SG_CUDA(cudaStreamSynchronize(h->stream));
-  return err ? fail(SG_ERR_TIMEOUT, "batched BFS: a grid barrier wait ran out") : SG_OK;
+  return h->report.finished() ? SG_OK : fail(SG_ERR_TIMEOUT, "batched BFS: a grid barrier wait ran out");
 }
 
 extern "C" {

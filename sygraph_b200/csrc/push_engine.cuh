@@ -17,6 +17,7 @@ struct PushLoop {
   Queues q;
   Counters* cnt;  // 3, zeroed before entry
   GridBarrier* bar;
+  ReportRef report;
   sg_level_record* log = nullptr;  // optional per-level log, entry log_base + level
   uint32_t log_base = 0;
 };

@@ -676,6 +676,7 @@ __global__ void __launch_bounds__(kThreads, 2) sssp_kernel(SsspParams<W> P) {
     P.result[1] = pass;
     P.result[2] = records;
     P.result[3] = phases;
+    report_run(P.L.report, total, pass, records, phases, 0);
   }
 }
 
@@ -722,7 +723,10 @@ __global__ void __launch_bounds__(kThreads, 2) cc_kernel(CcParams P) {
         return v;
       },
       s_scan, s_red);
-  if (gtid == 0) P.result[0] = levels;
+  if (gtid == 0 && levels) {  // (0: a barrier wait ran out)
+    P.result[0] = levels;
+    report_run(P.L.report, levels, 0, 0, 0, 0);
+  }
 }
 
 // Connected components of an undirected graph by lock-free union-find, then
@@ -803,6 +807,7 @@ struct UfParams {
   UfState* st;
   unsigned long long* result;
   GridBarrier* bar;
+  ReportRef report;
 };
 
 constexpr uint32_t kUfThreads = 1024, kUfSamples = kUfThreads;
@@ -974,7 +979,10 @@ __global__ void __launch_bounds__(kUfThreads, 2) uf_kernel(UfParams P) {
   if (threadIdx.x == 0 && s_giant_max) atomicMax(P.top + g, s_giant_max - 1);
   if (!grid_sync(P.bar)) return;
   for (uint32_t v = gtid; v < n; v += nthreads) parent[v] = ld_cg(P.top + ld_cg(parent + v));
-  if (gtid == 0) P.result[0] = 1;  // one pass over the edges (most skipped)
+  if (gtid == 0) {  // one pass over the edges (most skipped)
+    P.result[0] = 1;
+    report_run(P.report, 1, 0, 0, 0, 0);
+  }
 }
 
 }  // namespace
@@ -987,25 +995,31 @@ struct PushWorkspace {
   Counters* cnt = nullptr;
   GridBarrier* bar = nullptr;
   unsigned long long* result = nullptr;
+  RunReport report;
+  void* block = nullptr;  // the one device allocation behind the arrays above
   sg_status alloc(uint32_t n) {
     w0 = div_up(n, 32);
-    sg_status s;
-    if ((s = dev_alloc(&fb, 3ull * w0)) || (s = dev_alloc(&q.small, n)) || (s = dev_alloc(&q.big, n)) ||
-        (s = dev_alloc(&q.big_start, n)) || (s = dev_alloc(&cnt, 3)) || (s = dev_alloc(&bar, 1)) ||
-        (s = dev_alloc(&result, 4)))
-      return s;
-    return SG_OK;
+    Carve c;
+    const uint64_t afb = c.reserve(12ull * w0), asmall = c.reserve(4ull * n), abig = c.reserve(4ull * n),
+                   astart = c.reserve(4ull * n), acnt = c.reserve(3 * sizeof(Counters)),
+                   abar = c.reserve(sizeof(GridBarrier)), aresult = c.reserve(4 * sizeof(unsigned long long));
+    SG_TRY(dev_alloc(&c.base, c.bytes));
+    block = c.base;
+    fb = c.at<uint32_t>(afb);
+    q.small = c.at<uint32_t>(asmall);
+    q.big = c.at<uint32_t>(abig);
+    q.big_start = c.at<uint32_t>(astart);
+    cnt = c.at<Counters>(acnt);
+    bar = c.at<GridBarrier>(abar);
+    result = c.at<unsigned long long>(aresult);
+    return report.alloc();
   }
   void release() {
-    dev_free(fb);
-    dev_free(q.small);
-    dev_free(q.big);
-    dev_free(q.big_start);
-    dev_free(cnt);
-    dev_free(bar);
-    dev_free(result);
+    if (block) cudaFree(block);
+    block = nullptr;
+    report.release();
   }
-  PushLoop loop(sg_graph g) const {
+  PushLoop loop(sg_graph g) {
     PushLoop L;
     L.n = g->n;
     L.w0 = w0;
@@ -1015,16 +1029,13 @@ struct PushWorkspace {
     L.q = q;
     L.cnt = cnt;
     L.bar = bar;
+    L.report = report.next();
     return L;
   }
   sg_status finish(cudaStream_t s, uint64_t* levels) {
-    unsigned long long r = 0;
-    GridBarrier b;
-    SG_CUDA(cudaMemcpyAsync(&r, result, sizeof(r), cudaMemcpyDeviceToHost, s));
-    SG_CUDA(cudaMemcpyAsync(&b, bar, sizeof(b), cudaMemcpyDeviceToHost, s));
     SG_CUDA(cudaStreamSynchronize(s));
-    if (b.error) return fail(SG_ERR_TIMEOUT, "engine: a grid barrier wait ran out");
-    if (levels) *levels = r;
+    if (!report.finished()) return fail(SG_ERR_TIMEOUT, "engine: a grid barrier wait ran out");
+    if (levels) *levels = report.host->v[0];
     return SG_OK;
   }
 };
@@ -1301,10 +1312,7 @@ sg_status sg_sssp_level_features(sg_sssp s, float* host_features, uint32_t cap, 
 }  // extern "C"
 
 sg_status sgb::sssp_launch_status(sg_sssp s) {
-  uint32_t err = 0;
-  SG_CUDA(cudaMemcpyAsync(&err, &s->ws.bar->error, sizeof(err), cudaMemcpyDeviceToHost, s->stream));
-  SG_CUDA(cudaStreamSynchronize(s->stream));
-  return err ? fail(SG_ERR_TIMEOUT, "SSSP engine: a grid barrier wait ran out") : SG_OK;
+  return s->ws.finish(s->stream, nullptr);
 }
 
 extern "C" {
@@ -1458,7 +1466,7 @@ sg_status sg_cc_run_async(sg_cc_handle c) {
     static_assert(sizeof(UfState) <= 2 * sizeof(unsigned long long), "UfState lives in the last two result words");
     SG_CUDA(cudaMemsetAsync(c->ws.bar, 0, sizeof(GridBarrier), c->stream));
     UfParams P{g->fwd.ro, g->fwd.col, g->n, c->labels, c->ws.q.big, c->ws.q.small, c->ws.q.big_start,
-               reinterpret_cast<UfState*>(c->ws.result + 2), c->ws.result, c->ws.bar};
+               reinterpret_cast<UfState*>(c->ws.result + 2), c->ws.result, c->ws.bar, c->ws.report.next()};
     SG_TRY(launch_persistent(uf_kernel, P, 2, c->stream, (g->n - 1) / kUfThreads + 1, nullptr, kUfThreads));
   } else {
     SG_CUDA(cudaMemsetAsync(c->ws.bar, 0, sizeof(GridBarrier), c->stream));
