@@ -81,7 +81,7 @@ struct RowRange {
 };
 
 // Bitmap -> queues.  Each CTA owns a contiguous range of bitmap words and
-// takes them 32 words per warp: the warp ranks the set bits of its words and
+// takes them up to 32 words per warp: the warp ranks the set bits of its words and
 // every lane takes every 32nd rank, so the row-range loads of a dense word go
 // out together instead of one latency per set bit.  A first pass counts each
 // lane's vertices by class; one block scan and one atomic per list reserve
@@ -97,9 +97,16 @@ __device__ __forceinline__ void compact_frontier(const uint32_t* __restrict__ fb
   const uint32_t per_block = (w0 + gridDim.x - 1) / gridDim.x;
   const uint32_t wbeg = blockIdx.x * per_block;
   const uint32_t wend = min(w0, wbeg + per_block);
-  for (uint32_t base = wbeg; base < wend; base += blockDim.x) {
-    const uint32_t wi = base + threadIdx.x;
-    const uint32_t bits = wi < wend ? ld_cg(fb + wi) : 0u;
+  // words per warp and round: 32, or an even share where the CTA has fewer
+  // words than threads (graphs below 4.8 M vertices): with 32 a warp most warps
+  // had none and the others walked up to 1024 vertices in a chain (directed
+  // SSSP of 250 K vertices, 27 words a CTA: 317 -> 287 us)
+  const uint32_t nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  const uint32_t per_warp = min(32u, (per_block + nwarps - 1) / nwarps);
+  for (uint32_t base = wbeg; base < wend; base += nwarps * per_warp) {
+    const uint32_t w_first = base + warp * per_warp;  // the warp's first word
+    const uint32_t wi = w_first + lane;
+    const uint32_t bits = lane < per_warp && wi < wend ? ld_cg(fb + wi) : 0u;
     if (accumulate && bits) st_cg(accumulate + wi, ld_cg(accumulate + wi) | bits);
     // words all empty across the block (most blocks of a small frontier):
     // nothing to rank, count or reserve, so one barrier instead of the scans
@@ -108,7 +115,6 @@ __device__ __forceinline__ void compact_frontier(const uint32_t* __restrict__ fb
     const uint32_t incl = warp_inclusive_scan(c);
     const uint32_t total = __shfl_sync(kFullMask, incl, 31);
     const uint32_t excl = incl - c;
-    const uint32_t w_first = base + (threadIdx.x & ~31u);  // the warp's first word
     // vertex of rank r (< total) among the warp's set bits
     auto vertex_of = [&](uint32_t r) {
       const uint32_t o = warp_owner_of_rank(incl, r);
