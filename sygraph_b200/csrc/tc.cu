@@ -37,6 +37,7 @@ namespace sgb {
 namespace {
 
 using sygraph::detail::block_sum;
+using sygraph::detail::warp_owner_of_rank;
 
 constexpr uint32_t kTcThreads = 256, kTcWarps = kTcThreads / 32;
 constexpr uint32_t kTcBlocksPerSm = 5;  // 5 x 41 KB of shared memory, 48 registers
@@ -60,58 +61,83 @@ __device__ __forceinline__ bool dag_before(uint32_t du, uint32_t u, uint32_t dv,
   return du < dv || (du == dv && u < v);
 }
 
-// Keep bit of every edge, one thread per 32-edge word: the thread finds the
-// source of its first edge by binary search on the row offsets (kept in
-// wsrc for the compaction), loads the word's 32 columns and their 32 degrees
-// with every load in flight, then walks the rows.
+// Degrees of all vertices: the flags ask for one random word per edge instead
+// of two offsets.
+__global__ void __launch_bounds__(256) degree_kernel(const uint32_t* __restrict__ ro, uint32_t n,
+                                                     uint32_t* __restrict__ deg) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) deg[v] = ro[v + 1] - ro[v];
+}
+
+// Source of edge e0 + lane for the 32 edges of a word, given a row `first` at
+// or before the first one's: the row ends from there on, 32 at a time, ranked
+// by a warp search (rows without edges are passed over; lanes beyond the last
+// edge get its source).
+__device__ __forceinline__ uint32_t word_source(const uint32_t* __restrict__ ro, uint32_t n, uint32_t m, uint32_t first,
+                                                uint32_t e0) {
+  const uint32_t e = e0 + min(threadIdx.x & 31u, m - 1u - e0), lane = threadIdx.x & 31u;
+  uint32_t u = 0;
+  bool found = false;
+  for (uint32_t base = first;; base += 32) {
+    const uint32_t end = base + lane < n ? ro[base + lane + 1] : 0xffffffffu;
+    const uint32_t k = warp_owner_of_rank(end, e);  // of the first 31 ends, those at or below e
+    const uint32_t last = __shfl_sync(0xffffffffu, end, 31);
+    if (!found && last > e) {
+      u = base + k;
+      found = true;
+    }
+    if (__all_sync(0xffffffffu, found)) return u;
+  }
+}
+
+// Keep bit of every edge, a lane per edge: a warp takes up to kDagRun words in
+// a row, four at a time with their columns and degrees in flight, finds the
+// source of its first edge by a 32-ary search and goes on from row to row.
+// (One thread per word, with a binary search, 64 offset loads and a walk of
+// its own, took 284 us on RMAT-20; this form 229.)
+constexpr uint32_t kDagRun = 32, kDagWords = 4;
+
 __global__ void __launch_bounds__(256) dag_flags_kernel(const uint32_t* __restrict__ ro,
-                                                        const uint32_t* __restrict__ col, uint32_t n, uint32_t m,
+                                                        const uint32_t* __restrict__ col,
+                                                        const uint32_t* __restrict__ deg, uint32_t n, uint32_t m,
                                                         uint32_t nw, uint32_t* __restrict__ keep,
                                                         uint32_t* __restrict__ cnt, uint32_t* __restrict__ wsrc) {
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
   if (tid == 0) cnt[nw] = 0;  // the scan's last input: its output is the DAG size
-  for (uint32_t w = tid; w < nw; w += gridDim.x * blockDim.x) {
-    const uint32_t e0 = w * 32u, ne = (uint32_t)min((uint64_t)m - e0, (uint64_t)32u);
-    uint32_t v[32], dv[32];
-    if (ne == 32u) {  // col + e0 is 128-byte aligned
-      const uint4* c4 = reinterpret_cast<const uint4*>(col + e0);
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t run = min(kDagRun, max(kDagWords, nw / nwarps & ~(kDagWords - 1)));  // short where warps are left over
+  for (uint32_t w0 = (tid >> 5) * run; w0 < nw; w0 += nwarps * run) {
+    uint32_t row = 0, top = n;  // last row with ro[row] <= the first edge (ro[0] = 0)
+    while (top - row > 1) {
+      const uint32_t step = (top - row + 31) / 32, at = row + lane * step;
+      const uint32_t below = __ballot_sync(0xffffffffu, at < top && ro[at] <= w0 * 32u);
+      row += (31 - __clz(below)) * step;
+      top = min(top, row + step);
+    }
+    for (uint32_t w = w0; w < min(w0 + run, nw); w += kDagWords) {
+      uint32_t v[kDagWords], dv[kDagWords];
 #pragma unroll
-      for (uint32_t k = 0; k < 8; k++) {
-        const uint4 t = c4[k];
-        v[4 * k] = t.x;
-        v[4 * k + 1] = t.y;
-        v[4 * k + 2] = t.z;
-        v[4 * k + 3] = t.w;
+      for (uint32_t q = 0; q < kDagWords; q++) {
+        const uint64_t e = (uint64_t)(w + q) * 32u + lane;
+        v[q] = e < m ? col[e] : 0u;
       }
-    } else {
 #pragma unroll
-      for (uint32_t i = 0; i < 32; i++) v[i] = i < ne ? col[e0 + i] : 0u;
-    }
-    uint32_t lo = 0, hi = n - 1;  // last u with ro[u] <= e0: the source of edge e0
-    while (lo < hi) {
-      const uint32_t mid = lo + ((hi - lo + 1) >> 1);
-      if (ro[mid] <= e0)
-        lo = mid;
-      else
-        hi = mid - 1;
-    }
+      for (uint32_t q = 0; q < kDagWords; q++) dv[q] = deg[v[q]];
 #pragma unroll
-    for (uint32_t i = 0; i < 32; i++) dv[i] = i < ne ? ro[v[i] + 1] - ro[v[i]] : 0u;
-    wsrc[w] = lo;
-    uint32_t u = lo, rb = ro[u], re = ro[u + 1], bits = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < 32; i++) {
-      if (i < ne) {
-        while (re <= e0 + i) {  // rows without edges are skipped
-          u++;
-          rb = re;
-          re = ro[u + 1];
+      for (uint32_t q = 0; q < kDagWords; q++) {
+        if (w + q >= nw) break;  // uniform
+        const uint32_t e0 = (w + q) * 32u;
+        const uint32_t u = word_source(ro, n, m, row, e0);
+        const bool in = (uint64_t)e0 + lane < m;
+        const uint32_t bits = __ballot_sync(0xffffffffu, in && dag_before(deg[u], u, dv[q], v[q]));
+        row = __shfl_sync(0xffffffffu, u, 0);
+        if (lane == 0) {
+          keep[w + q] = bits;
+          cnt[w + q] = __popc(bits);
+          wsrc[w + q] = row;
         }
-        if (dag_before(re - rb, u, dv[i], v[i])) bits |= 1u << i;
+        row = __shfl_sync(0xffffffffu, u, 31);
       }
     }
-    keep[w] = bits;
-    cnt[w] = __popc(bits);
   }
 }
 
@@ -122,51 +148,65 @@ __device__ __forceinline__ uint32_t dag_prefix(const uint32_t* keep, const uint3
 }
 
 // Stable compaction of the kept edges into the DAG's columns (and each
-// edge's source) and the DAG's row offsets; zeroes the reverse counts.
+// edge's source), a lane per edge, and the DAG's row offsets and out-degrees;
+// zeroes the reverse counts.  (One thread per word walked its bits one by one:
+// 372 us on RMAT-20; this form 147.)
 __global__ void __launch_bounds__(256) dag_fill_kernel(const uint32_t* __restrict__ ro, const uint32_t* __restrict__ col,
-                                                       uint32_t n, uint32_t nw, const uint32_t* __restrict__ keep,
+                                                       uint32_t n, uint32_t m, uint32_t nw,
+                                                       const uint32_t* __restrict__ keep,
                                                        const uint32_t* __restrict__ wpre,
                                                        const uint32_t* __restrict__ wsrc, uint32_t* __restrict__ dro,
-                                                       uint32_t* __restrict__ dcol, uint32_t* __restrict__ dsrc,
-                                                       uint32_t* __restrict__ rcnt) {
+                                                       uint32_t* __restrict__ ddeg, uint32_t* __restrict__ dcol,
+                                                       uint32_t* __restrict__ dsrc, uint32_t* __restrict__ rcnt) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-  for (uint32_t w = tid; w < nw; w += nthreads) {
-    uint32_t bits = keep[w], p = wpre[w];
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t w = tid >> 5; w < nw; w += nthreads >> 5) {
+    const uint32_t bits = keep[w];
     if (!bits) continue;
-    const uint32_t e0 = w * 32u;
-    uint32_t u = wsrc[w], re = ro[u + 1];
-    while (bits) {
-      const uint32_t j = __ffs(bits) - 1u;
-      bits &= bits - 1u;
-      while (re <= e0 + j) re = ro[++u + 1];  // rows without edges are skipped
-      dcol[p] = col[e0 + j];
-      dsrc[p++] = u;
+    const uint32_t p = wpre[w], e0 = w * 32u;
+    const bool on = (bits >> lane) & 1u;
+    const uint32_t c = on ? col[e0 + lane] : 0u;
+    const uint32_t u = word_source(ro, n, m, wsrc[w], e0);
+    if (on) {
+      const uint32_t at = p + __popc(bits & ((1u << lane) - 1u));
+      dcol[at] = c;
+      dsrc[at] = u;
     }
   }
   for (uint32_t u = tid; u <= n; u += nthreads) {
-    dro[u] = dag_prefix(keep, wpre, ro[u]);
+    const uint32_t b = dag_prefix(keep, wpre, ro[u]);
+    dro[u] = b;
+    if (u < n) ddeg[u] = dag_prefix(keep, wpre, ro[u + 1]) - b;
     rcnt[u] = 0;
   }
 }
 
 // The reverse lists: for every DAG edge y -> x with d+(y) < d+(x), y joins
 // x's list (the edge's shorter row N+(y) is then streamed against x's set).
-// One thread per DAG edge; kFill = false counts, kFill = true places (rcnt
-// counted down to zero).
-template <bool kFill>
-__global__ void __launch_bounds__(256) rev_kernel(const uint32_t* __restrict__ dro, const uint32_t* __restrict__ dcol,
-                                                  const uint32_t* __restrict__ dsrc, const uint32_t* dm_ptr,
-                                                  uint32_t* __restrict__ rcnt, const uint32_t* __restrict__ rro,
-                                                  uint32_t* __restrict__ rcol) {
+// One thread per DAG edge: the count takes its place in x's list, the fill
+// writes there (each pass with its own offsets and atomics: 221 + 305 us on
+// RMAT-20; with the out-degrees in one array and the places kept 234 + 122).
+constexpr uint32_t kNoPlace = 0xffffffffu;
+
+__global__ void __launch_bounds__(256) rev_count_kernel(const uint32_t* __restrict__ ddeg,
+                                                        const uint32_t* __restrict__ dcol,
+                                                        const uint32_t* __restrict__ dsrc, const uint32_t* dm_ptr,
+                                                        uint32_t* __restrict__ rcnt, uint32_t* __restrict__ place) {
   const uint32_t dm = *dm_ptr;  // DAG edges
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < dm; i += gridDim.x * blockDim.x) {
-    const uint32_t y = dsrc[i], x = dcol[i];
-    if (dro[y + 1] - dro[y] < dro[x + 1] - dro[x]) {
-      if (kFill)
-        rcol[rro[x] + atomicSub(rcnt + x, 1u) - 1u] = y;
-      else
-        atomicAdd(rcnt + x, 1u);
-    }
+    const uint32_t x = dcol[i];
+    place[i] = ddeg[dsrc[i]] < ddeg[x] ? atomicAdd(rcnt + x, 1u) : kNoPlace;
+  }
+}
+
+__global__ void __launch_bounds__(256) rev_fill_kernel(const uint32_t* __restrict__ dcol,
+                                                       const uint32_t* __restrict__ dsrc, const uint32_t* dm_ptr,
+                                                       const uint32_t* __restrict__ place,
+                                                       const uint32_t* __restrict__ rro, uint32_t* __restrict__ rcol) {
+  const uint32_t dm = *dm_ptr;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < dm; i += gridDim.x * blockDim.x) {
+    const uint32_t at = place[i];
+    if (at != kNoPlace) rcol[rro[dcol[i]] + at] = dsrc[i];
   }
 }
 
@@ -541,6 +581,8 @@ struct sg_tc_s {
   uint32_t* dro = nullptr;   // n + 1
   uint32_t* dcol = nullptr;  // up to m
   uint32_t* dsrc = nullptr;  // up to m
+  uint32_t* deg = nullptr;   // n: degrees for the flags, then the DAG's out-degrees
+  uint32_t* place = nullptr; // up to m: each DAG edge's place in its head's reverse list
   uint32_t* rcnt = nullptr;  // n + 1
   uint32_t* rro = nullptr;   // n + 1
   uint32_t* rcol = nullptr;  // up to m
@@ -565,6 +607,8 @@ sg_status sg_tc_destroy(sg_tc_handle t) {
     dev_free(t->dro);
     dev_free(t->dcol);
     dev_free(t->dsrc);
+    dev_free(t->deg);
+    dev_free(t->place);
     dev_free(t->rcnt);
     dev_free(t->rro);
     dev_free(t->rcol);
@@ -591,7 +635,7 @@ sg_status sg_tc_create(sg_graph g, sg_tc_handle* out) {
   if ((st = dev_alloc(&t->keep, t->nw)) || (st = dev_alloc(&t->wsrc, t->nw)) || (st = dev_alloc(&t->cnt, (uint64_t)t->nw + 1)) ||
       (st = dev_alloc(&t->wpre, (uint64_t)t->nw + 1)) ||
       (st = dev_alloc(&t->tiles, div_up((uint64_t)t->nw + 1, kScanTile))) || (st = dev_alloc(&t->dro, n + 1)) ||
-      (st = dev_alloc(&t->dcol, m)) || (st = dev_alloc(&t->dsrc, m)) || (st = dev_alloc(&t->rcnt, n + 1)) || (st = dev_alloc(&t->rro, n + 1)) ||
+      (st = dev_alloc(&t->dcol, m)) || (st = dev_alloc(&t->dsrc, m)) || (st = dev_alloc(&t->deg, n)) || (st = dev_alloc(&t->place, m)) || (st = dev_alloc(&t->rcnt, n + 1)) || (st = dev_alloc(&t->rro, n + 1)) ||
       (st = dev_alloc(&t->rcol, m)) || (st = dev_alloc(&t->rtiles, div_up(n + 1, kScanTile))) ||
       (st = dev_alloc(&t->lists, 3 * n)) || (st = dev_alloc(&t->counters, 1))) {
     sg_tc_destroy(t);
@@ -609,24 +653,25 @@ sg_status sg_tc_run_async(sg_tc_handle t, int per_vertex) {
   cudaStream_t s = t->stream;
   if (per_vertex && !t->pv) SG_TRY(dev_alloc(&t->pv, n));
   SG_CUDA(cudaMemsetAsync(t->counters, 0, sizeof(TcCounters), s));
-  dag_flags_kernel<<<grid_for(t->nw ? t->nw : 1, 256, 8), 256, 0, s>>>(g->fwd.ro, g->fwd.col, n, m, t->nw, t->keep,
-                                                                       t->cnt, t->wsrc);
+  degree_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(g->fwd.ro, n, t->deg);
+  dag_flags_kernel<<<grid_for(8ull * t->nw + 1, 256, 8), 256, 0, s>>>(
+      g->fwd.ro, g->fwd.col, t->deg, n, m, t->nw, t->keep, t->cnt, t->wsrc);
   SG_CUDA(cudaGetLastError());
-  count_launch();
+  count_launch(2);
   SG_TRY(exclusive_scan_u32(t->cnt, t->nw + 1, t->wpre, t->tiles, s));
   const unsigned vgrid = grid_for((uint64_t)n + 1, 256, 8), egrid = grid_for(m ? m : 1, 256, 8);
-  dag_fill_kernel<<<grid_for(std::max<uint64_t>(t->nw, (uint64_t)n + 1), 256, 8), 256, 0, s>>>(
-      g->fwd.ro, g->fwd.col, n, t->nw, t->keep, t->wpre, t->wsrc, t->dro, t->dcol, t->dsrc, t->rcnt);
+  dag_fill_kernel<<<grid_for(std::max<uint64_t>(32ull * t->nw, (uint64_t)n + 1), 256, 8), 256, 0, s>>>(
+      g->fwd.ro, g->fwd.col, n, m, t->nw, t->keep, t->wpre, t->wsrc, t->dro, t->deg, t->dcol, t->dsrc, t->rcnt);
   SG_CUDA(cudaGetLastError());
   count_launch();
   if (t->shorter) {  // the DAG size is read on the device: dro[n]
-    rev_kernel<false><<<egrid, 256, 0, s>>>(t->dro, t->dcol, t->dsrc, t->dro + n, t->rcnt, nullptr, nullptr);
+    rev_count_kernel<<<egrid, 256, 0, s>>>(t->deg, t->dcol, t->dsrc, t->dro + n, t->rcnt, t->place);
     SG_CUDA(cudaGetLastError());
     count_launch();
   }
   SG_TRY(exclusive_scan_u32(t->rcnt, n + 1, t->rro, t->rtiles, s));
   if (t->shorter) {
-    rev_kernel<true><<<egrid, 256, 0, s>>>(t->dro, t->dcol, t->dsrc, t->dro + n, t->rcnt, t->rro, t->rcol);
+    rev_fill_kernel<<<egrid, 256, 0, s>>>(t->dcol, t->dsrc, t->dro + n, t->place, t->rro, t->rcol);
     SG_CUDA(cudaGetLastError());
     count_launch();
   }
