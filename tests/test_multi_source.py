@@ -149,3 +149,23 @@ def test_msbfs_forced_and_learned_schedules_keep_depths(sg, oracle, rmat, scale,
     assert asked >= 2
     mb.set_selector(None)
     mb.log_features(False)
+
+
+@pytest.mark.parametrize("n", [31, 33, 127, 1025, 5000, 40_001])
+@pytest.mark.parametrize("degree", [1, 6])
+def test_batch_dense_and_sparse_folds(sg, oracle, n, degree):
+    """Frontiers on both sides of the dense fold's limit (n / 512 vertices),
+    vertex counts around a word and a warp's four words, shallow and deep
+    graphs (up to several depth planes)."""
+    rng = np.random.default_rng(n + degree)
+    path = np.arange(n - 1)
+    s = np.concatenate([path[:: degree + 1], rng.integers(0, n, degree * n)])
+    d = np.concatenate([path[:: degree + 1] + 1, (s[len(path[:: degree + 1]):] + rng.integers(1, 40, degree * n)) % n])
+    g = sg.io.fromCOO(n, s, d, symmetrize=True, dedupe=True, drop_self_loops=True)
+    mb = sg.algorithms.MultiBFS(sg.graph.build.fromCSR(g), 64)
+    for k in (1, 17, 64):
+        src = rng.integers(0, n, k).astype(np.uint32)
+        mb.run(src, 2, 4.0, 24.0)
+        got = mb.getDistances()
+        for i in range(k):
+            assert np.array_equal(got[i], oracle.bfs_levels(g, int(src[i])))
