@@ -190,61 +190,69 @@ __global__ void __launch_bounds__(kKeepThreads) row_fill_kernel(uint32_t* __rest
 // values.  The fill also checks whether the weighted adjacency is symmetric
 // (each row strictly increasing in column, every edge's reverse present with
 // the same weight), which the pull phases of delta-stepping need.
-constexpr uint32_t kWsBig = 256;  // rows at least this long are filled by a whole warp
-
+//
+// Of the two edges between u and v it is the one towards the smaller end (by
+// degree, then id) whose reverse is looked up, by a binary search of the
+// smaller row; where all of those have theirs and there are as many edges
+// towards the larger end, every edge has.
 struct WsortParams {
   const uint32_t* ro;
   const uint32_t* col;
   const uint32_t* val;
-  uint32_t n;
+  uint32_t n, m;
   u64* k0;
   uint32_t* v0;
-  uint32_t* big;        // rows of at least kWsBig edges (n entries)
-  uint32_t* big_count;
-  uint32_t* asym;       // set when the adjacency is not symmetric with sorted rows
+  uint32_t* asym;       // set when a row is not increasing or a reverse is missing
+  u64* towards;         // edges towards their smaller end, and towards their larger one
 };
 
-// Edge i of row v: its sort pair, and whether it breaks symmetry.
-__device__ __forceinline__ bool ws_edge(const WsortParams& P, uint32_t v, uint32_t i, uint32_t e) {
-  const uint32_t u = P.col[i], w = P.val[i];
-  P.k0[i] = ((u64)v << 32) | w;
-  P.v0[i] = u;
-  if (i + 1 < e && u >= P.col[i + 1]) return true;
-  uint32_t lo = P.ro[u], hi = P.ro[u + 1];  // v in row u (sorted): lower bound
-  const uint32_t end = hi;
-  while (lo < hi) {
-    const uint32_t mid = lo + ((hi - lo) >> 1);
-    if (P.col[mid] < v)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo == end || P.col[lo] != v || P.val[lo] != w;
-}
+// A warp takes up to kWsRun runs of 32 edges in a row, a lane per edge.  (A thread
+// per short row and a warp per long one took 10 ms on RMAT-22 and another 42
+// for its largest hub; this form 6.)
+constexpr uint32_t kWsRun = 32;
 
-// Short rows, one thread each; long rows are listed for whole warps.
 __global__ void __launch_bounds__(256) ws_fill_kernel(WsortParams P) {
+  __shared__ u64 s_red[32];
+  const uint32_t lane = threadIdx.x & 31u, words = (P.m - 1) / 32 + 1;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t run = min(kWsRun, max(1u, words / nwarps));
   bool bad = false;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < P.n; v += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t b = P.ro[v], e = P.ro[v + 1];
-    if (e - b >= kWsBig) {
-      P.big[atomicAdd(P.big_count, 1u)] = (uint32_t)v;
-      continue;
+  u64 smaller = 0, larger = 0;
+  for (uint32_t w0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * run; w0 < words; w0 += nwarps * run) {
+    uint32_t row = eng::row_of_edge(P.ro, P.n, w0 * 32u);
+    for (uint32_t w = w0; w < min(w0 + run, words); w++) {
+      const uint32_t e0 = w * 32u;
+      const uint32_t v = eng::word_source(P.ro, P.n, P.m, row, e0);
+      row = __shfl_sync(kFullMask, v, 31);
+      if (lane > P.m - 1u - e0) continue;  // the last word; no collective follows in this turn
+      const uint32_t i = e0 + lane, u = P.col[i], x = P.val[i];
+      P.k0[i] = ((u64)v << 32) | x;
+      P.v0[i] = u;
+      const uint32_t vb = P.ro[v], ve = P.ro[v + 1], end = P.ro[u + 1];
+      uint32_t lo = P.ro[u], hi = end;
+      if (i + 1 < ve && u >= P.col[i + 1]) bad = true;
+      const uint32_t dv = ve - vb, du = end - lo;
+      if (du > dv || (du == dv && u > v)) {
+        larger++;
+      } else if (u != v) {
+        smaller++;
+        while (lo < hi) {  // v in row u (sorted): lower bound
+          const uint32_t mid = lo + ((hi - lo) >> 1);
+          if (P.col[mid] < v)
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
+        if (lo == end || P.col[lo] != v || P.val[lo] != x) bad = true;
+      }
     }
-    for (uint32_t i = b; i < e; i++) bad |= ws_edge(P, (uint32_t)v, i, e);
   }
   if (bad) *P.asym = 1u;
-}
-
-__global__ void __launch_bounds__(256) ws_fill_big_kernel(WsortParams P) {
-  const uint32_t nbig = *P.big_count, lane = threadIdx.x & 31u;
-  bool bad = false;
-  for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < nbig; j += (gridDim.x * blockDim.x) >> 5) {
-    const uint32_t v = P.big[j];
-    const uint32_t b = P.ro[v], e = P.ro[v + 1];
-    for (uint64_t i = (uint64_t)b + lane; i < e; i += 32) bad |= ws_edge(P, v, (uint32_t)i, e);
+  const u64 a = sygraph::detail::block_sum<u64>(smaller, s_red), b = sygraph::detail::block_sum<u64>(larger, s_red);
+  if (threadIdx.x == 0) {
+    if (a) atomicAdd(P.towards, a);
+    if (b) atomicAdd(P.towards + 1, b);
   }
-  if (bad) *P.asym = 1u;
 }
 
 __global__ void __launch_bounds__(256) low_words_kernel(const u64* __restrict__ key, uint64_t m,
@@ -273,8 +281,8 @@ sg_status graph_weight_sorted(sg_graph g) {
   cudaStream_t st = g->stream;
   const uint32_t bits = 32 + bit_length(n - 1), passes = (bits + 7) / 8;
   Carve c;
-  const uint64_t k0 = c.reserve(8 * ma), k1 = c.reserve(8 * ma), v = c.reserve(4 * ma), big = c.reserve(4ull * n),
-                 words = c.reserve(4 * 3), scratch = c.reserve(4 * rsort::scratch_words(m));
+  const uint64_t k0 = c.reserve(8 * ma), k1 = c.reserve(8 * ma), v = c.reserve(4 * ma), words = c.reserve(24),
+                 scratch = c.reserve(4 * rsort::scratch_words(m));
   uint32_t *wc = nullptr, *wv = nullptr;
   sg_status s = SG_OK;
   do {
@@ -282,24 +290,27 @@ sg_status graph_weight_sorted(sg_graph g) {
     u64* k[2] = {c.at<u64>(k0), c.at<u64>(k1)};
     uint32_t* vals[2] = {c.at<uint32_t>(v), c.at<uint32_t>(v)};
     vals[passes & 1] = wc;  // the sorted columns stay where the last pass puts them
-    uint32_t* flags = c.at<uint32_t>(words);  // long rows, asymmetric, m
-    const gb::WsortParams P{g->fwd.ro, g->fwd.col, reinterpret_cast<const uint32_t*>(g->fwd.val),
-                            n,         k[0],       vals[0], c.at<uint32_t>(big), flags, flags + 1};
-    const uint32_t init[3] = {0, 0, (uint32_t)m};
-    cudaError_t e = cudaMemcpyAsync(flags, init, sizeof(init), cudaMemcpyHostToDevice, st);
+    struct {
+      u64 towards[2];
+      uint32_t asym, m;
+    } flags = {{0, 0}, 0, (uint32_t)m};
+    static_assert(sizeof(flags) == 24, "reserved above");
+    char* dev = c.at<char>(words);
+    const gb::WsortParams P{g->fwd.ro,  g->fwd.col, reinterpret_cast<const uint32_t*>(g->fwd.val),
+                            n,          (uint32_t)m, k[0], vals[0], reinterpret_cast<uint32_t*>(dev + 16),
+                            reinterpret_cast<u64*>(dev)};
+    cudaError_t e = cudaMemcpyAsync(dev, &flags, sizeof(flags), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && m) {
-      gb::ws_fill_kernel<<<grid_for(n, 256, 8), 256, 0, st>>>(P);
-      gb::ws_fill_big_kernel<<<device_props().sm_count * 8, 256, 0, st>>>(P);
-      count_launch(2);
+      gb::ws_fill_kernel<<<grid_for((m - 1) / 32 + 1, 8, 8), 256, 0, st>>>(P);
+      count_launch();
       uint32_t done, *left;
-      const rsort::ArraySource src{k[0], vals[0], flags + 2};
+      const rsort::ArraySource src{k[0], vals[0], reinterpret_cast<uint32_t*>(dev + 20)};
       if ((s = rsort::sort_pairs(src, m, bits, k, vals, c.at<uint32_t>(scratch), st, &done, &left)) != SG_OK) break;
       gb::low_words_kernel<<<grid_for(m, 256, 8), 256, 0, st>>>(k[passes & 1], m, wv);
       e = cudaGetLastError();
       count_launch();
     }
-    uint32_t hf[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, dev, sizeof(flags), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
       s = cuda_fail(e, "weight sort", __FILE__, __LINE__);
@@ -308,7 +319,7 @@ sg_status graph_weight_sorted(sg_graph g) {
     g->wcol = wc;
     g->wval = wv;
     wc = wv = nullptr;
-    g->wsym = hf[1] == 0;
+    g->wsym = flags.asym == 0 && flags.towards[0] == flags.towards[1];
     g->bytes += 8ull * m;
   } while (0);
   dev_free(c.base);

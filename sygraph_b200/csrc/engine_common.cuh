@@ -205,6 +205,41 @@ __device__ __forceinline__ uint32_t warp_find_owner(const uint32_t* start, uint3
   return lo;
 }
 
+// Last row with ro[row] <= e (the row of edge e, or an empty one before it):
+// a warp-wide 32-ary search.  Called by the whole warp with one e.
+__device__ __forceinline__ uint32_t row_of_edge(const uint32_t* __restrict__ ro, uint32_t n, uint32_t e) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t row = 0, top = n;  // ro[0] = 0
+  while (top - row > 1) {
+    const uint32_t step = (top - row + 31) / 32, at = row + lane * step;
+    const uint32_t below = __ballot_sync(kFullMask, at < top && ro[at] <= e);
+    row += (31 - __clz(below)) * step;
+    top = min(top, row + step);
+  }
+  return row;
+}
+
+// Source of edge e0 + lane for the 32 edges of a word, given a row `first` at
+// or before the first one's: the row ends from there on, 32 at a time, ranked
+// by a warp search (rows without edges are passed over; lanes beyond the last
+// edge get its source).
+__device__ __forceinline__ uint32_t word_source(const uint32_t* __restrict__ ro, uint32_t n, uint32_t m, uint32_t first,
+                                                uint32_t e0) {
+  const uint32_t e = e0 + min(threadIdx.x & 31u, m - 1u - e0), lane = threadIdx.x & 31u;
+  uint32_t u = 0;
+  bool found = false;
+  for (uint32_t base = first;; base += 32) {
+    const uint32_t end = base + lane < n ? ro[base + lane + 1] : 0xffffffffu;
+    const uint32_t k = warp_owner_of_rank(end, e);  // of the first 31 ends, those at or below e
+    const uint32_t last = __shfl_sync(0xffffffffu, end, 31);
+    if (!found && last > e) {
+      u = base + k;
+      found = true;
+    }
+    if (__all_sync(0xffffffffu, found)) return u;
+  }
+}
+
 // Degree-bucketed push expansion over the queues of one frontier.  Work units
 // are 32-vertex groups of small vertices (edge-parallel inside the warp by a
 // shuffle scan) and kChunk-edge chunks of big vertices; warps take units

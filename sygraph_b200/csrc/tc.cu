@@ -31,7 +31,7 @@
 // is counted in pieces of 1024 keys, each piece against all of x's rows.  The count is that of a graph without parallel
 // edges (the reference's sorted-list merge assumes none either); self-loops
 // are no DAG edges.
-#include "internal.cuh"
+#include "engine_common.cuh"
 
 namespace sgb {
 namespace {
@@ -68,27 +68,6 @@ __global__ void __launch_bounds__(256) degree_kernel(const uint32_t* __restrict_
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) deg[v] = ro[v + 1] - ro[v];
 }
 
-// Source of edge e0 + lane for the 32 edges of a word, given a row `first` at
-// or before the first one's: the row ends from there on, 32 at a time, ranked
-// by a warp search (rows without edges are passed over; lanes beyond the last
-// edge get its source).
-__device__ __forceinline__ uint32_t word_source(const uint32_t* __restrict__ ro, uint32_t n, uint32_t m, uint32_t first,
-                                                uint32_t e0) {
-  const uint32_t e = e0 + min(threadIdx.x & 31u, m - 1u - e0), lane = threadIdx.x & 31u;
-  uint32_t u = 0;
-  bool found = false;
-  for (uint32_t base = first;; base += 32) {
-    const uint32_t end = base + lane < n ? ro[base + lane + 1] : 0xffffffffu;
-    const uint32_t k = warp_owner_of_rank(end, e);  // of the first 31 ends, those at or below e
-    const uint32_t last = __shfl_sync(0xffffffffu, end, 31);
-    if (!found && last > e) {
-      u = base + k;
-      found = true;
-    }
-    if (__all_sync(0xffffffffu, found)) return u;
-  }
-}
-
 // Keep bit of every edge, a lane per edge: a warp takes up to kDagRun words in
 // a row, four at a time with their columns and degrees in flight, finds the
 // source of its first edge by a 32-ary search and goes on from row to row.
@@ -106,13 +85,7 @@ __global__ void __launch_bounds__(256) dag_flags_kernel(const uint32_t* __restri
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t run = min(kDagRun, max(kDagWords, nw / nwarps & ~(kDagWords - 1)));  // short where warps are left over
   for (uint32_t w0 = (tid >> 5) * run; w0 < nw; w0 += nwarps * run) {
-    uint32_t row = 0, top = n;  // last row with ro[row] <= the first edge (ro[0] = 0)
-    while (top - row > 1) {
-      const uint32_t step = (top - row + 31) / 32, at = row + lane * step;
-      const uint32_t below = __ballot_sync(0xffffffffu, at < top && ro[at] <= w0 * 32u);
-      row += (31 - __clz(below)) * step;
-      top = min(top, row + step);
-    }
+    uint32_t row = eng::row_of_edge(ro, n, w0 * 32u);
     for (uint32_t w = w0; w < min(w0 + run, nw); w += kDagWords) {
       uint32_t v[kDagWords], dv[kDagWords];
 #pragma unroll
@@ -126,7 +99,7 @@ __global__ void __launch_bounds__(256) dag_flags_kernel(const uint32_t* __restri
       for (uint32_t q = 0; q < kDagWords; q++) {
         if (w + q >= nw) break;  // uniform
         const uint32_t e0 = (w + q) * 32u;
-        const uint32_t u = word_source(ro, n, m, row, e0);
+        const uint32_t u = eng::word_source(ro, n, m, row, e0);
         const bool in = (uint64_t)e0 + lane < m;
         const uint32_t bits = __ballot_sync(0xffffffffu, in && dag_before(deg[u], u, dv[q], v[q]));
         row = __shfl_sync(0xffffffffu, u, 0);
@@ -166,7 +139,7 @@ __global__ void __launch_bounds__(256) dag_fill_kernel(const uint32_t* __restric
     const uint32_t p = wpre[w], e0 = w * 32u;
     const bool on = (bits >> lane) & 1u;
     const uint32_t c = on ? col[e0 + lane] : 0u;
-    const uint32_t u = word_source(ro, n, m, wsrc[w], e0);
+    const uint32_t u = eng::word_source(ro, n, m, wsrc[w], e0);
     if (on) {
       const uint32_t at = p + __popc(bits & ((1u << lane) - 1u));
       dcol[at] = c;

@@ -42,3 +42,35 @@ def test_weight_sorted_rows(sg, rmat, kind):
     assert np.array_equal(col, want_col)
     assert np.array_equal(val.view(np.uint32), want_val.view(np.uint32))
     assert sym == kind.startswith(("rmat", "grid"))
+
+
+@pytest.mark.parametrize("n", [2, 33, 500])
+@pytest.mark.parametrize("broken", ["none", "missing", "weight", "both_missing", "self_loop"])
+def test_weight_symmetry_flag(sg, n, broken):
+    """The flag looks one direction of every pair up and counts the other: a
+    reverse missing towards either end, a weight that differs, and self-loops
+    (their own reverse)."""
+    rng = np.random.default_rng(n)
+    a = np.arange(n - 1)
+    s, d = np.concatenate([a, np.zeros(n - 1, int)]), np.concatenate([a + 1, a + 1])  # a path and a star on 0
+    pairs = sorted({(min(x, y), max(x, y)) for x, y in zip(s, d)})
+    w = rng.integers(1, 50, len(pairs))
+    edges = {(x, y): k for (x, y), k in zip(pairs, w)} | {(y, x): k for (x, y), k in zip(pairs, w)}
+    if broken == "missing":  # towards the larger end (vertex 0) of one pair
+        del edges[(pairs[-1][1], pairs[-1][0])]
+    elif broken == "both_missing" and len(pairs) > 1:  # one towards each end, of different pairs
+        del edges[pairs[0]]
+        del edges[(pairs[-1][1], pairs[-1][0])]
+    elif broken == "weight":
+        edges[pairs[0]] += 1
+    elif broken == "self_loop":
+        edges[(n // 2, n // 2)] = 7
+    e = sorted(edges)
+    ro = np.searchsorted([x for x, _ in e], np.arange(n + 1)).astype(np.uint32)
+    g = sg.CSR(ro, np.array([y for _, y in e], np.uint32), np.array([edges[x] for x in e], np.uint32))
+    G = sg.graph.build.fromCSR(g)
+    col, val, sym = G.weight_sorted()
+    want_col, want_val = host_sorted(g)
+    assert np.array_equal(col, want_col) and np.array_equal(val, want_val)
+    bits = {(x, y): k for (x, y), k in edges.items()}
+    assert sym == all(bits.get((y, x)) == k for (x, y), k in bits.items())
