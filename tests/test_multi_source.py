@@ -169,3 +169,25 @@ def test_batch_dense_and_sparse_folds(sg, oracle, n, degree):
         got = mb.getDistances()
         for i in range(k):
             assert np.array_equal(got[i], oracle.bfs_levels(g, int(src[i])))
+
+
+@pytest.mark.parametrize("k", [1, 2, 33, 64])
+def test_batch_repeated_and_heavy_sources(sg, oracle, rmat, k):
+    """Repeated sources share a vertex, a hub (a heavy frontier vertex) among
+    them; totals count every source, the frontier a vertex once."""
+    g = rmat(12, perm_seed=3)
+    hub = int(np.argmax(g.degrees()))
+    src = np.resize(np.array([hub, int(sg.io.sample_sources(g, 1, seed=9)[0]), hub, 0], np.uint32), k)
+    G = sg.graph.build.fromCSR(g)
+    mb = sg.algorithms.MultiBFS(G, 64)
+    bc = sg.algorithms.BatchedBC(G)
+    det = mb.run(src, 2, 4.0, 24.0)
+    got = mb.getDistances()
+    deg = g.degrees().astype(np.int64)
+    want = {int(s): oracle.bfs_levels(g, int(s)) for s in set(src.tolist())}
+    for i, s in enumerate(src):
+        assert np.array_equal(got[i], want[int(s)])
+    assert det["reached_edges"] == sum(int(deg[want[int(s)] <= g.n].sum()) for s in src)
+    bc.run(src)
+    ref = oracle.bc(g, src)
+    assert np.allclose(bc.getBC(), ref, rtol=1e-4, atol=1e-6 * max(1.0, float(ref.max())))
