@@ -219,23 +219,6 @@ __global__ void __launch_bounds__(kBfsThreads, 2) bfs_kernel(Params P) {
     P.result[3] = visited_vertices;
     P.result[4] = P.m - unexplored;
   }
-  if (blockIdx.x == 0 && P.report.at) {
-    // the step bits, from the log that this block's thread 0 kept
-    __syncthreads();
-    const uint32_t steps = min(level + 1, kMaxLog);
-    for (uint32_t i = threadIdx.x; i < (steps + 31u & ~31u); i += blockDim.x) {
-      const uint32_t w = __ballot_sync(kFullMask, i < steps && ld_cg(&P.log[i].strategy) >= 2u);
-      if ((i & 31u) == 0) {
-        *const_cast<volatile uint32_t*>(P.report.at->pull + (i >> 5)) = w;
-        __threadfence_system();
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // (this thread wrote the results)
-      const volatile unsigned long long* r = P.result;
-      report_run(P.report, r[0], r[1], r[2], r[3], r[4]);
-    }
-  }
   {
     // n+1 for every vertex not reached: reached = visited, minus the vertices
     // pre-marked for having no in-edge, plus the source.  Four vertices per
@@ -313,7 +296,7 @@ struct sg_bfs_s {
   sygraph::detail::GridBarrier* bar = nullptr;
   sg_level_record* log = nullptr;
   unsigned long long* result = nullptr;
-  eng::RunReport report;
+  char* host_tail = nullptr;  // pinned copy of the barrier, the results and the first log records
   void* block = nullptr;  // the one device allocation behind the arrays above
   int* schedule = nullptr;
   uint32_t schedule_len = 0;
@@ -348,7 +331,7 @@ static sg_status bfs_materialise(sg_bfs b) {
 static void bfs_release(sg_bfs b) {
   if (!b) return;
   if (b->block) cudaFree(b->block);
-  b->report.release();
+  pinned_give(b->host_tail);
   dev_free(b->schedule);
   dev_free(b->features);
   delete b;
@@ -395,7 +378,6 @@ static sg_status bfs_launch(sg_bfs b, int direction, float alpha, float beta) {
   P.bar = b->bar;
   P.log = b->log;
   P.result = b->result;
-  P.report = b->report.next();
   P.schedule = b->schedule_len ? b->schedule : nullptr;
   P.schedule_len = b->schedule_len;
   if (b->bar_reset) {
@@ -405,23 +387,46 @@ static sg_status bfs_launch(sg_bfs b, int direction, float alpha, float beta) {
   return eng::launch_persistent(bfs::bfs_kernel, P, 2, b->stream, b->max_ctas, nullptr, bfs::kBfsThreads);
 }
 
-static sg_status bfs_collect(sg_bfs b, sg_bfs_details* details) {
+// The barrier, the results and the log's first records lie together and come
+// back in one copy to pinned memory (two or three pageable copies, each with a
+// wait of its own, took 25 us longer).  The kernel does not write them there
+// itself, as the other engines do: with that code at its end the compiler made
+// its push levels 2% slower.
+constexpr size_t kTailResult = 64, kTailLog = 128;
+constexpr uint32_t kTailRecords = (uint32_t)((kPinnedPiece - kTailLog) / sizeof(sg_level_record));
+
+static sg_status bfs_read_tail(sg_bfs b, size_t bytes) {
+  SG_CUDA(cudaMemcpyAsync(b->host_tail, b->bar, bytes, cudaMemcpyDeviceToHost, b->stream));
   SG_CUDA(cudaStreamSynchronize(b->stream));
-  if (!b->report.finished()) {
+  if (reinterpret_cast<const sygraph::detail::GridBarrier*>(b->host_tail)->error) {
     b->bar_reset = true;
     return fail(SG_ERR_TIMEOUT, "BFS engine: a grid barrier wait ran out");
   }
-  const unsigned long long* res = b->report.host->v;
+  return SG_OK;
+}
+
+static sg_status bfs_collect(sg_bfs b, sg_bfs_details* details) {
+  SG_TRY(bfs_read_tail(b, details ? kPinnedPiece : kTailLog));
+  const unsigned long long* res = reinterpret_cast<const unsigned long long*>(b->host_tail + kTailResult);
   b->last_iterations = (uint32_t)res[0];
   if (details) {
+    memset(details, 0, sizeof(*details));
     details->iterations = res[0];
     details->push_steps = res[1];
     details->pull_steps = res[2];
     details->visited_vertices = res[3];
     details->visited_edges = res[4];
     const uint32_t nlog = res[0] < SG_MAX_LOGGED_LEVELS ? (uint32_t)res[0] : SG_MAX_LOGGED_LEVELS;
-    memset(details->step_is_pull, 0, SG_MAX_LOGGED_LEVELS);
-    for (uint32_t i = 0; i < nlog; i++) details->step_is_pull[i] = (b->report.host->pull[i >> 5] >> (i & 31)) & 1u;
+    const sg_level_record* first = reinterpret_cast<const sg_level_record*>(b->host_tail + kTailLog);
+    for (uint32_t i = 0; i < nlog && i < kTailRecords; i++) details->step_is_pull[i] = first[i].strategy >= 2;
+    if (nlog > kTailRecords) {
+      // (a std::vector of this C struct trips an internal error of nvcc 12.9's
+      // front end under -std=c++20)
+      const uint32_t more = nlog - kTailRecords;
+      std::unique_ptr<sg_level_record[]> recs(new sg_level_record[more]);
+      SG_CUDA(cudaMemcpy(recs.get(), b->log + kTailRecords, sizeof(sg_level_record) * more, cudaMemcpyDeviceToHost));
+      for (uint32_t i = 0; i < more; i++) details->step_is_pull[kTailRecords + i] = recs[i].strategy >= 2;
+    }
   }
   return SG_OK;
 }
@@ -445,11 +450,15 @@ sg_status sg_bfs_create(sg_graph g, sg_bfs* out) {
   const uint64_t depth = c.reserve(4 * n), visited = c.reserve(4ull * b->w0), fb = c.reserve(12ull * b->w0),
                  sm = c.reserve(12ull * b->w1), no_in = c.reserve(4ull * b->w0), first_in = c.reserve(4 * n),
                  heavy_v = c.reserve(8ull * b->heavy_cap), heavy_s = c.reserve(8ull * b->heavy_cap),
-                 cnt = c.reserve(3 * sizeof(bfs::LevelCounters)), bar = c.reserve(sizeof(*b->bar)),
-                 log = c.reserve(SG_MAX_LOGGED_LEVELS * sizeof(sg_level_record)), result = c.reserve(8 * 8);
+                 cnt = c.reserve(3 * sizeof(bfs::LevelCounters)),
+                 tail = c.reserve(kTailLog + SG_MAX_LOGGED_LEVELS * sizeof(sg_level_record));
+  static_assert(sizeof(sygraph::detail::GridBarrier) <= kTailResult && kTailResult + 8 * 8 <= kTailLog, "tail layout");
   sg_status s = dev_alloc(&c.base, c.bytes);
   b->block = c.base;
-  if (s != SG_OK || (s = b->report.alloc()) != SG_OK) {
+  void* piece = nullptr;
+  if (s == SG_OK) s = pinned_take(&piece);
+  b->host_tail = static_cast<char*>(piece);
+  if (s != SG_OK) {
     bfs_release(b);
     return s;
   }
@@ -462,9 +471,9 @@ sg_status sg_bfs_create(sg_graph g, sg_bfs* out) {
   b->heavy_v = c.at<uint32_t>(heavy_v);
   b->heavy_s = c.at<uint32_t>(heavy_s);
   b->cnt = c.at<bfs::LevelCounters>(cnt);
-  b->bar = c.at<sygraph::detail::GridBarrier>(bar);
-  b->log = c.at<sg_level_record>(log);
-  b->result = c.at<unsigned long long>(result);
+  b->bar = c.at<sygraph::detail::GridBarrier>(tail);
+  b->log = c.at<sg_level_record>(tail + kTailLog);
+  b->result = c.at<unsigned long long>(tail + kTailResult);
   bfs::no_in_edges_kernel<<<grid_for((uint64_t)b->w0 * 32, 256), 256, 0, g->stream>>>(g->inv.ro, g->n, b->w0,
                                                                                        b->no_in);
   bfs::first_in_kernel<<<grid_for(n, 256), 256, 0, g->stream>>>(g->inv.ro, g->inv.col, g->n, b->first_in);
@@ -543,10 +552,7 @@ sg_status sg_bfs_set_schedule(sg_bfs b, const int* host_strategies, uint32_t len
 }  // extern "C"
 
 sg_status sgb::bfs_launch_status(sg_bfs b) {
-  SG_CUDA(cudaStreamSynchronize(b->stream));
-  if (b->report.finished()) return SG_OK;
-  b->bar_reset = true;
-  return fail(SG_ERR_TIMEOUT, "BFS engine: a grid barrier wait ran out");
+  return bfs_read_tail(b, kTailLog);
 }
 
 extern "C" {

@@ -75,7 +75,6 @@ struct Params {
   unsigned long long pull_reverse;        // bit L: level L's pull probes in-neighbours from the back
   uint32_t pull_words;                    // short-circuit pull: 0 ranked candidates, or 2 / 4 words per warp step
   float* features;                        // optional log: 12 floats per level decision
-  ReportRef report;
 };
 
 struct Shared {

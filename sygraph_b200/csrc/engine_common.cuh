@@ -325,7 +325,6 @@ __device__ __forceinline__ uint32_t valid_bits(uint32_t wi, uint32_t w0, uint32_
 struct HostReport {
   unsigned long long v[5];
   unsigned long long run;
-  uint32_t pull[kMaxLog / 32];  // BFS: bit i % 32 of word i / 32 = step i pulled
 };
 struct ReportRef {
   HostReport* at = nullptr;  // null: nobody reads one
