@@ -273,7 +273,9 @@ typedef struct {
  *   expected_size : SG_SIZE_FETCH_FROM_MEMORY, SG_SIZE_INFER_FROM_DEVICE or a
  *     positive hint.  The active-word count is always read on the device, so
  *     none of them costs a host round trip.
- * Pull directions walk the inverse graph (common.hpp:147). */
+ * Pull directions walk the inverse graph (common.hpp:147).
+ * `in` and `out` may be the same frontier; each candidate is then tested once,
+ * but a test may see what the call has inserted by then. */
 sg_status sg_advance(sg_graph g, sg_frontier in, sg_frontier out, int direction, int load_balancer, int in_view,
                      int out_view, int op, const sg_op_args* args, int expected_size);
 

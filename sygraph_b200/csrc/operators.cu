@@ -160,9 +160,13 @@ sg_status sg_advance(sg_graph g, sg_frontier in, sg_frontier out, int direction,
     SG_TRY(frontier_compact(in, direction != SG_DIR_PUSH, s));
   }
   if (out_view == SG_VIEW_VERTEX) a.out = mlb_dev(out);
-  const GraphDir& dir = direction != SG_DIR_PUSH ? g->inv : g->fwd;
-  a.hub_units = dir.hub_units;
-  a.n_hub_units = dir.n_hub_units;
+  // A unit's candidate is tested when the unit is walked, which must not see
+  // what this advance inserts: long rows are in units where the frontiers differ.
+  if (in_view != SG_VIEW_VERTEX || out_view != SG_VIEW_VERTEX || in != out) {
+    const GraphDir& dir = direction != SG_DIR_PUSH ? g->inv : g->fwd;
+    a.hub_units = dir.hub_units;
+    a.n_hub_units = dir.n_hub_units;
+  }
   const sg_graph_view v = g->view(direction != SG_DIR_PUSH);
   return dispatch(op, x, direction, load_balancer, v, a, advance_grid(expected_size), s);
 }

@@ -282,3 +282,27 @@ def test_advance_long_rows(sg, ops, lb, directed):
                 assert np.array_equal(fout.flags(), reference_advance(ro, col, flags, direction))
                 fout.clear()
                 assert fout.empty() and fout.size() == 0
+
+
+@pytest.mark.parametrize("lb", [2, 3])
+def test_advance_in_place_long_row(sg, ops, lb):
+    """One frontier as input and output: a long row's candidate is decided
+    once, whatever its first edges insert (pull_all), and a long row that the
+    advance itself inserts is no candidate of it (push)."""
+    deg = 600_000  # more units than a CTA looks at together
+    n = deg + 1
+    g = sg.CSR(np.concatenate([[0], deg + np.arange(n)]).astype(np.uint32),
+               np.concatenate([np.arange(1, n), np.zeros(deg)]).astype(np.uint32))
+    G = sg.graph.build.fromCSR(g)
+    leaves = np.arange(1, n)
+    for direction, active in ((2, leaves), (0, leaves[-1:])):
+        f = sg.frontier.makeFrontier(G)
+        f.insert_list(active)
+        visits = sg.DeviceArray(np.zeros(n, np.uint32))
+        ops.advance.frontier(G, f, f, ops.OP_COUNT_VISITS, ops.op_args([visits]), direction, lb, expected_size=1)
+        want = np.zeros(n, np.uint32)
+        want[0 if direction == 2 else n - 1] = active.size
+        assert np.array_equal(visits.numpy(), want)
+        flags = np.zeros(n, np.uint8)
+        flags[active] = flags[0] = 1
+        assert np.array_equal(f.flags(), flags)
