@@ -582,7 +582,11 @@ sg_status sg_run_sssp(sg_graph g, uint32_t source, void* host_dist, uint64_t* it
  * union-find in the Afforest order (sampled neighbours until one component
  * dominates, then the other edges of the vertices outside it) followed by
  * the largest id of each component (SG_CC_UNION_FIND): the same labels.
- * SG_CC_AUTO picks union-find for undirected graphs. */
+ * SG_CC_AUTO picks union-find for undirected graphs.
+ * Either method is one cooperative launch of up to the whole GPU: it starts
+ * when all of its CTAs fit beside what other streams run, and a wait in it
+ * that runs out is SG_ERR_TIMEOUT from sg_cc_run, or, after sg_cc_run_async,
+ * from sg_cc_get_labels (whoever reads the device array is not told). */
 #define SG_CC_AUTO 0
 #define SG_CC_PROPAGATION 1
 #define SG_CC_UNION_FIND 2

@@ -1486,9 +1486,14 @@ sg_status sg_cc_get_labels(sg_cc_handle c, uint32_t* host_labels) {
   clear_error();
   SG_REQUIRE(c && host_labels, SG_ERR_INVALID, "NULL argument");
   SG_REQUIRE(c->ran, SG_ERR_NOT_INITIALIZED, "CC not run");
+  // after a run that was only enqueued this is where its outcome is first
+  // looked at; the barrier itself is asked, which a replay of a captured run
+  // sets too (its report has the number of the capture)
+  GridBarrier bar;
   SG_CUDA(cudaMemcpyAsync(host_labels, c->labels, sizeof(uint32_t) * c->g->n, cudaMemcpyDeviceToHost, c->stream));
+  SG_CUDA(cudaMemcpyAsync(&bar, c->ws.bar, sizeof(bar), cudaMemcpyDeviceToHost, c->stream));
   SG_CUDA(cudaStreamSynchronize(c->stream));
-  return SG_OK;
+  return bar.error ? fail(SG_ERR_TIMEOUT, "CC engine: a grid barrier wait ran out") : SG_OK;
 }
 
 sg_status sg_cc_labels_device(sg_cc_handle c, const uint32_t** dev_labels) {

@@ -30,3 +30,13 @@ def test_cpp_api_known_answers(golden):
     print(r.stdout)
     assert r.returncode == 0, r.stderr
     assert "ALL OK" in r.stdout
+
+
+def test_status_of_unfinished_runs():
+    """tests/cpp/run_status.cu: what a run that gave up at a grid barrier
+    leaves behind, and what the calls that follow make of it."""
+    b = _build_module()
+    b.build_library()
+    exe = {p.name: p for p in b.build_cpp_tests()}["run_status"]
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "ALL OK" in r.stdout, r.stderr
