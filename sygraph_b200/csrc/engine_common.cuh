@@ -319,8 +319,8 @@ __device__ __forceinline__ uint32_t valid_bits(uint32_t wi, uint32_t w0, uint32_
 }
 
 // What a run leaves in pinned host memory for the host to read when the stream
-// is idle: its totals, and last its number, without which it did not finish
-// (a barrier wait ran out).  Two or three small copies from the device, each
+// is idle: its totals, and its number, without which it did not finish (a
+// barrier wait ran out).  Two or three small copies from the device, each
 // about 8 us with its wait, were a third of a small graph's run.
 struct HostReport {
   unsigned long long v[5];
@@ -331,17 +331,23 @@ struct ReportRef {
   unsigned long long run = 0;
 };
 
-__device__ __forceinline__ void report_run(const ReportRef& r, unsigned long long a, unsigned long long b,
-                                           unsigned long long c, unsigned long long d, unsigned long long e) {
-  if (!r.at) return;
-  volatile unsigned long long* v = r.at->v;
-  v[0] = a;
-  v[1] = b;
-  v[2] = c;
-  v[3] = d;
-  v[4] = e;
-  __threadfence_system();
-  *reinterpret_cast<volatile unsigned long long*>(&r.at->run) = r.run;
+// Called by every block that is past its last barrier: block 0 leaves the
+// totals (the same in all), and the last block out the number, so a run that
+// any block gave up, at its last barrier too, has none.  Counts in the
+// barrier's `exits`, which the host clears with the barrier for each launch.
+__device__ __forceinline__ void report_run(const ReportRef& r, GridBarrier* bar, unsigned long long a,
+                                           unsigned long long b, unsigned long long c, unsigned long long d,
+                                           unsigned long long e) {
+  if (!r.at || threadIdx.x) return;
+  if (blockIdx.x == 0) {
+    volatile unsigned long long* v = r.at->v;
+    v[0] = a;
+    v[1] = b;
+    v[2] = c;
+    v[3] = d;
+    v[4] = e;
+  }
+  if (atomicAdd(&bar->exits, 1u) == gridDim.x - 1) *reinterpret_cast<volatile unsigned long long*>(&r.at->run) = r.run;
 }
 
 // The host's side, one per instance.

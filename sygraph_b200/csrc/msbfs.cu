@@ -717,8 +717,8 @@ __global__ void __launch_bounds__(kThreads, 2) msbfs_kernel(Params P) {
     P.result[1] = n_push;
     P.result[2] = n_pull;
     P.result[3] = reached_total;
-    report_run(P.report, level + 1, n_push, n_pull, reached_total, 0);
   }
+  report_run(P.report, P.bar, level + 1, n_push, n_pull, reached_total, 0);
 }
 
 __global__ void no_in_edges_kernel(const uint32_t* __restrict__ iro, uint32_t n, uint32_t w0, uint32_t* out) {

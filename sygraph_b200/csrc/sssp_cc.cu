@@ -676,8 +676,8 @@ __global__ void __launch_bounds__(kThreads, 2) sssp_kernel(SsspParams<W> P) {
     P.result[1] = pass;
     P.result[2] = records;
     P.result[3] = phases;
-    report_run(P.L.report, total, pass, records, phases, 0);
   }
+  report_run(P.L.report, P.L.bar, total, pass, records, phases, 0);
 }
 
 struct CcParams {
@@ -723,10 +723,9 @@ __global__ void __launch_bounds__(kThreads, 2) cc_kernel(CcParams P) {
         return v;
       },
       s_scan, s_red);
-  if (gtid == 0 && levels) {  // (0: a barrier wait ran out)
-    P.result[0] = levels;
-    report_run(P.L.report, levels, 0, 0, 0, 0);
-  }
+  if (!levels) return;  // a barrier wait ran out
+  if (gtid == 0) P.result[0] = levels;
+  report_run(P.L.report, P.L.bar, levels, 0, 0, 0, 0);
 }
 
 // Connected components of an undirected graph by lock-free union-find, then
@@ -979,10 +978,8 @@ __global__ void __launch_bounds__(kUfThreads, 2) uf_kernel(UfParams P) {
   if (threadIdx.x == 0 && s_giant_max) atomicMax(P.top + g, s_giant_max - 1);
   if (!grid_sync(P.bar)) return;
   for (uint32_t v = gtid; v < n; v += nthreads) parent[v] = ld_cg(P.top + ld_cg(parent + v));
-  if (gtid == 0) {  // one pass over the edges (most skipped)
-    P.result[0] = 1;
-    report_run(P.report, 1, 0, 0, 0, 0);
-  }
+  if (gtid == 0) P.result[0] = 1;  // one pass over the edges (most skipped)
+  report_run(P.report, P.bar, 1, 0, 0, 0, 0);
 }
 
 }  // namespace

@@ -1,5 +1,7 @@
-// Status of a run whose grid barrier gave up.  Nothing here waits for a block
-// that does not come: the barrier's error word is set by a memset.
+// Status of a run whose grid barrier gave up: what a launch leaves behind for
+// the host, and what the host makes of it.  Nothing here waits for a block
+// that does not come: a block that "gave up" returns, and the barrier's error
+// word is set by a copy.
 #include "sssp_cc.cu"
 
 #include <cstdio>
@@ -12,6 +14,34 @@
       std::exit(1);                                                             \
     }                                                                           \
   } while (0)
+
+// A run whose block `leaves` stops at its last barrier.
+__global__ void run_kernel(eng::ReportRef report, sygraph::detail::GridBarrier* bar, uint32_t leaves) {
+  if (!sygraph::detail::grid_sync(bar)) return;
+  if (blockIdx.x == leaves) return;
+  eng::report_run(report, bar, 1, 2, 3, 4, 5);
+}
+
+static void report_needs_every_block() {
+  eng::RunReport report;
+  EXPECT(report.alloc() == SG_OK);
+  sygraph::detail::GridBarrier* bar = nullptr;
+  EXPECT(cudaMalloc(&bar, sizeof(*bar)) == cudaSuccess);
+  const uint32_t blocks = 8;
+  for (uint32_t leaves : {blocks, 0u, 1u, blocks, 7u, blocks}) {
+    eng::ReportRef ref = report.next();
+    uint32_t who = leaves;
+    void* args[] = {&ref, &bar, &who};
+    EXPECT(cudaMemset(bar, 0, sizeof(*bar)) == cudaSuccess);
+    EXPECT(cudaLaunchCooperativeKernel((const void*)run_kernel, dim3(blocks), dim3(64), args, 0, 0) == cudaSuccess);
+    EXPECT(cudaDeviceSynchronize() == cudaSuccess);
+    EXPECT(report.finished() == (leaves == blocks));
+    if (leaves == blocks)
+      for (uint32_t i = 0; i < 5; i++) EXPECT(report.host->v[i] == i + 1);
+  }
+  report.release();
+  cudaFree(bar);
+}
 
 // Labels are not handed out after a run that gave up, with either method, and
 // are after the next run; replays of a captured run do not confuse the status.
@@ -51,6 +81,7 @@ static void labels_of_an_unfinished_run() {
 
 int main() {
   labels_of_an_unfinished_run();
+  report_needs_every_block();
   std::puts("ALL OK");
   return 0;
 }
