@@ -1,6 +1,8 @@
 """Triangle counting and connected components through their instances, against
 the oracle: block-table vertices (DAG out-degree above 128), unsorted rows,
 self-loops, graphs without edges, and repeated runs."""
+import time
+
 import numpy as np
 import pytest
 
@@ -225,3 +227,24 @@ def test_cc_union_find_hub_outside_giant(sg, oracle, hub_degree, giant):
     for _ in range(3):
         cc.run()
         assert np.array_equal(cc.getLabels(), ref)
+
+
+@pytest.mark.parametrize("gap", [0, 31, 200, 12_000_000])
+def test_tc_across_empty_rows(sg, gap):
+    """A clique whose ids leave a long run of vertices without edges, inside a
+    word of 32 edges: the same count, and no time spent on the run."""
+    k, half = 80, 40
+    n = k + 12_000_000
+    ids = np.concatenate([np.arange(half), half + gap + np.arange(half)])
+    deg = np.zeros(n, np.int64)
+    deg[ids] = k - 1
+    ro = np.concatenate([[0], np.cumsum(deg)]).astype(np.uint32)
+    i, j = np.nonzero(~np.eye(k, dtype=bool))
+    tc = sg.algorithms.TC(sg.graph.build.fromCSR(sg.CSR(ro, ids[j].astype(np.uint32))))
+    seconds = []
+    for _ in range(3):
+        t = time.perf_counter()
+        tc.run()
+        seconds.append(time.perf_counter() - t)
+        assert tc.getNumTriangles() == k * (k - 1) * (k - 2) // 6
+    assert min(seconds) < 0.05

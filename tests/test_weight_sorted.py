@@ -2,6 +2,8 @@
 (sg_graph_weight_sorted): every row holds the same (column, weight) pairs as
 the CSR, in non-decreasing weight order with equal weights in column order,
 and the symmetry flag is right."""
+import time
+
 import numpy as np
 import pytest
 
@@ -74,3 +76,27 @@ def test_weight_symmetry_flag(sg, n, broken):
     assert np.array_equal(col, want_col) and np.array_equal(val, want_val)
     bits = {(x, y): k for (x, y), k in edges.items()}
     assert sym == all(bits.get((y, x)) == k for (x, y), k in bits.items())
+
+
+@pytest.mark.parametrize("gap", [0, 31, 200, 12_000_000])
+def test_weight_sorted_rows_across_empty_rows(sg, gap):
+    """Long runs of vertices without edges, inside and between the words of 32
+    edges that a warp takes: the same rows, and no time spent on the run (a
+    warp that passes it 32 rows at a time takes 0.15 s for the longest one)."""
+    k, half = 80, 40
+    n = k + 12_000_000
+    ids = np.concatenate([np.arange(half), half + gap + np.arange(half)])
+    deg = np.zeros(n, np.int64)
+    deg[ids] = k - 1
+    ro = np.concatenate([[0], np.cumsum(deg)]).astype(np.uint32)
+    i, j = np.nonzero(~np.eye(k, dtype=bool))
+    g = sg.CSR(ro, ids[j].astype(np.uint32), (1 + (i * j) % 7).astype(np.uint32))
+    want_col, want_val = host_sorted(g)
+    seconds = []
+    for _ in range(3):
+        G = sg.graph.build.fromCSR(g)
+        t = time.perf_counter()
+        col, val, sym = G.weight_sorted()
+        seconds.append(time.perf_counter() - t)
+        assert np.array_equal(col, want_col) and np.array_equal(val, want_val) and sym
+    assert min(seconds) < 0.05
