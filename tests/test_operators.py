@@ -2,6 +2,8 @@
 tests (tests/operators/*.cpp, tests/frontier/mlb_frontier.cpp) ported through
 the C ABI, plus randomised checks of every direction x load balancer against
 a Python restatement of the advance semantics (operators/advance/common.hpp:49-75)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -306,3 +308,29 @@ def test_advance_in_place_long_row(sg, ops, lb):
         flags = np.zeros(n, np.uint8)
         flags[active] = flags[0] = 1
         assert np.array_equal(f.flags(), flags)
+
+
+@pytest.mark.parametrize("lb", [2, 3])
+def test_advance_size_hint_with_many_long_rows(sg, ops, lb):
+    """A small size hint gives a small grid; on a graph with many long rows it
+    costs no more than the default does."""
+    hubs, deg = 40_000, 512
+    n = hubs + 1000
+    ro = np.minimum(np.arange(n + 1, dtype=np.int64), hubs) * deg
+    col = (np.arange(hubs * deg, dtype=np.uint32) % deg) + np.uint32(hubs)
+    G = sg.graph.build.fromCSR(sg.CSR(ro.astype(np.uint32), col))
+    fin, fout = sg.frontier.makeFrontier(G), sg.frontier.makeFrontier(G)
+    fin.insert_list(np.array([3, n - 1]))
+    visits = sg.DeviceArray(np.zeros(n, np.uint32))
+    best = {}
+    for hint in (sg.operators.size.fetch_from_memory, 1):
+        for _ in range(4):
+            t = time.perf_counter()
+            for _ in range(50):
+                ops.advance.frontier(G, fin, fout, ops.OP_COUNT_VISITS, ops.op_args([visits]), 0, lb,
+                                     expected_size=hint)
+            assert fout.size() == deg
+            best[hint] = min(best.get(hint, 1.0), time.perf_counter() - t)
+    got = visits.numpy()
+    assert got[3] == 2 * 4 * 50 * deg and got.sum() == got[3]
+    assert best[1] < 3 * best[sg.operators.size.fetch_from_memory] + 1e-3
