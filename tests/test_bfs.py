@@ -140,3 +140,37 @@ def test_bfs_consecutive_runs_across_components(sg, oracle, directed):
             bfs.getDistances()  # the initial state, written before the run
         bfs.run(sg.algorithms.bfs_direction.hybrid, 15.0, 24.0)
         assert np.array_equal(bfs.getDistances(), oracle.bfs_levels(g, s0)), (directed, s0)
+
+
+@pytest.mark.parametrize("levels", [1, 15, 16, 17, 18, 60, 500])
+def test_bfs_step_directions_deep(sg, levels):
+    """push_steps / pull_steps of runs with few and with many levels: a path
+    from its end, its directions forced in an irregular order."""
+    n = levels
+    v = np.arange(n - 1)
+    g = sg.io.fromCOO(n, v, v + 1, symmetrize=True)
+    b = sg.algorithms.BFS(sg.graph.build.fromCSR(g))
+    pulls = np.random.default_rng(levels).random(levels) < 0.5
+    b.set_schedule(np.where(pulls, 2, 0))
+    for _ in range(2):
+        b.init(0)
+        det = b.run(sg.algorithms.bfs_direction.hybrid, 15.0, 24.0)
+        assert det.iterations == levels
+        assert det.pull_steps == set(np.nonzero(pulls)[0].tolist())
+        assert det.push_steps == set(np.nonzero(~pulls)[0].tolist())
+        assert np.array_equal(b.getDistances(), np.arange(n))
+
+
+def test_bfs_step_directions_deep_hybrid(sg, oracle):
+    """Hybrid runs of a grid with long-range pairs (dozens of levels, both
+    directions) against the oracle's steps."""
+    for side, frac in ((60, 0.0), (120, 0.002), (200, 0.001)):
+        g = sg.io.grid(side, frac)
+        b = sg.algorithms.BFS(sg.graph.build.fromCSR(g))
+        b.init(0)
+        det = b.run(sg.algorithms.bfs_direction.hybrid, 15.0, 24.0)
+        ref, it, steps = oracle.bfs_frontier(g, 0, 2, 15.0, 24.0)
+        assert it > 16 and det.iterations == it
+        assert det.pull_steps == {i for i, p in enumerate(steps) if p}
+        assert det.push_steps == {i for i, p in enumerate(steps) if not p}
+        assert np.array_equal(b.getDistances(), ref)
