@@ -100,7 +100,9 @@ struct AdvanceArgs {
 // Rows that a CTA does not walk alone.  On an RMAT graph of 300 K vertices one
 // CTA walked a hub's 100 K edges 256 at a time while the others had finished:
 // 206 us for that level's advance, 67 with the rows in units.
-// Below 512 edges a row is two rounds of its CTA; a unit is four.
+// Below 512 edges a row is two rounds of its CTA; a unit is four.  The list is
+// looked through whatever the frontier holds: an advance of one vertex takes
+// 10.3 us with its compaction instead of 9.2 (RMAT-18).
 constexpr uint32_t kHubDegree = 512, kHubUnit = 1024;
 
 // The units of the candidates among the long rows, spread over the grid: a

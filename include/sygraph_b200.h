@@ -645,7 +645,7 @@ sg_status sg_bc_batched(sg_graph g, const uint32_t* host_sources, uint32_t k, fl
  * have no parallel edges (self-loops are ignored).
  * getNumTriangles(v), the per-vertex count, is for every edge (u,v) with
  * u < v, |N(u) n N(v)| added to u.  The instance owns the DAG, its reverse
- * lists and the work lists (about 12m + 32n bytes), so that runs allocate
+ * lists and the work lists (about 16.5m + 28n bytes), so that runs allocate
  * nothing; runs are enqueued on the graph's stream. */
 typedef struct sg_tc_s* sg_tc_handle;
 sg_status sg_tc_create(sg_graph g, sg_tc_handle* out);

@@ -413,9 +413,10 @@ __global__ void __launch_bounds__(kThreads, 2) bc_batch_kernel(Params P) {
   }
   if (!grid_sync(P.bar)) return;
   // ---- sources: depth 0, sigma 1; high-degree sources go on the level-0 mark
-  // list; a thread per source (one thread for all of them, three round trips
-  // each, cost 64 sources on RMAT-20 0.17 of 10.05 ms).  The counters were
-  // zeroed above.
+  // list; a thread per source.  (One thread for all of them, three round
+  // trips each, cost 64 sources about 0.1 ms whatever the graph: 1.93 -> 1.84
+  // ms on RMAT-10; on RMAT-20, 10 ms, it is within the noise of the runs.)
+  // The counters were zeroed above.
   if (gtid < P.k) {
     const uint32_t s = P.sources[gtid];
     const u64 bit = 1ull << gtid;

@@ -58,8 +58,7 @@ struct EdgeSource {
 // its run of equal keys, or every entry without de-duplication).
 constexpr uint32_t kKeepThreads = 512, kKeepItems = 8, kKeepTile = kKeepThreads * kKeepItems;
 
-// Bit r: entry base + 32 r + lane is kept; `before`: the warp's kept entries
-// of the earlier lanes' and rounds' entries are counted by the caller.
+// Bit r: entry base + 32 r is kept; `base` is the lane's first entry.
 __device__ __forceinline__ uint32_t keep_bits(const u64* __restrict__ key, uint32_t count, int dedupe, uint64_t base) {
   uint32_t bits = 0;
 #pragma unroll

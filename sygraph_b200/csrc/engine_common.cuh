@@ -100,7 +100,7 @@ __device__ __forceinline__ void compact_frontier(const uint32_t* __restrict__ fb
   // words per warp and round: 32, or an even share where the CTA has fewer
   // words than threads (graphs below 4.8 M vertices): with 32 a warp most warps
   // had none and the others walked up to 1024 vertices in a chain (directed
-  // SSSP of 250 K vertices, 27 words a CTA: 317 -> 287 us)
+  // SSSP of 250 K vertices, 27 words a CTA: 312 -> 266 us with the report)
   const uint32_t nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5;
   const uint32_t per_warp = min(32u, (per_block + nwarps - 1) / nwarps);
   for (uint32_t base = wbeg; base < wend; base += nwarps * per_warp) {

@@ -140,12 +140,12 @@ struct GraphDir {
   void* val = nullptr;
   void* block = nullptr;  // the one allocation behind all of it, where they share one
   // long rows in units for the operators' advances (advance_kernels.cuh): the
-  // count, and hub_units(count) as (vertex, first edge)
+  // count, and that many units as (vertex, first edge)
   uint32_t* n_hub_units = nullptr;
   uint2* hub_units = nullptr;
 };
 
-// Bytes of a direction's unit list (at most m / kHubUnit full units and one
+// Entries of a direction's unit list (at most m / kHubUnit full units and one
 // more for each of at most m / kHubDegree rows), and its build on the device.
 uint64_t hub_units_capacity(uint64_t m);
 sg_status build_hub_units(GraphDir& d, uint32_t n, cudaStream_t stream);

@@ -354,7 +354,8 @@ __global__ void __launch_bounds__(kThreads, 2) msbfs_kernel(Params P) {
   if (!grid_sync(P.bar)) return;
   // ---- sources: F_0, seen, depth 0, and the level-0 heavy list; a thread per
   // source (one thread for all of them was a chain of 64 x three round trips,
-  // 64 sources on RMAT-20: 724 -> 667 us).  The counters were zeroed above.
+  // 64 sources on RMAT-20: 724 -> 667 us; RMAT-10 0.41 -> 0.22 ms with the dense
+  // fold and the report).  The counters were zeroed above.
   if (gtid < P.k) {
     const uint32_t s = P.sources[gtid];
     const u64 bit = 1ull << gtid;
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(kThreads, 2) msbfs_kernel(Params P) {
       // each plane's words in flight together.  (A summary word per warp, its
       // 32 fa words one after the other, left most warps of a graph below
       // 2^22 vertices idle and the others 32 chains of three round trips:
-      // 64 sources on RMAT-20 939 -> 770 us with this form)
+      // 64 sources on RMAT-20 932 -> 749 us with this form)
       const uint32_t dprev = level - 1;
       for (uint32_t w = gwarp * kFoldWords; w < w0; w += nwarps * kFoldWords) {
         uint32_t word[kFoldWords];

@@ -887,7 +887,8 @@ __device__ __forceinline__ void uf_pick_giant(const UfParams& P) {
 // roots: RMAT of 3.0 M vertices with shuffled ids took 153 ms when a hub that
 // the sampled links had missed was one thread's work, 0.92 ms with its rows
 // cut but a find and a CAS per sampled edge (all of them end on one address
-// in the L2), 0.27 ms in this form; RMAT-22 0.42 ms -> 0.17 ms.  The phases are
+// in the L2), 0.19-0.27 ms (by the box) in this form; RMAT-22 0.42 ms -> 0.17
+// ms.  The phases are
 // one launch because the rounds that a graph does not need cost nothing there
 // (nine empty launches are 20 us, a third of the time on RMAT-10).
 __global__ void __launch_bounds__(kUfThreads, 2) uf_kernel(UfParams P) {
