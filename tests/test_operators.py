@@ -334,3 +334,29 @@ def test_advance_size_hint_with_many_long_rows(sg, ops, lb):
     got = visits.numpy()
     assert got[3] == 2 * 4 * 50 * deg and got.sum() == got[3]
     assert best[1] < 3 * best[sg.operators.size.fetch_from_memory] + 1e-3
+
+
+@pytest.mark.parametrize("lb", [2, 3])
+def test_advance_long_rows_with_small_hint(sg, ops, lb):
+    """Every edge of a candidate's long row exactly once (push, pull_all) from
+    the grid of a small size hint too, with more units than it has blocks."""
+    degs = [511, 512, 1025, 2049] + [3000] * 400
+    n = 6000
+    rng = np.random.default_rng(23)
+    s = np.concatenate([np.full(d, h) for h, d in enumerate(degs)])
+    d = np.concatenate([rng.choice(np.arange(500, n), k, replace=False) for k in degs])
+    g = sg.io.fromCOO(n, s, d, symmetrize=True, dedupe=True)
+    G = sg.graph.build.fromCSR(g)
+    ro, col = g.row_offsets, g.column_indices
+    flags = (rng.random(n) < 0.5).astype(np.uint8)
+    for direction in (0, 2):
+        fin, fout = sg.frontier.makeFrontier(G), sg.frontier.makeFrontier(G)
+        fin.insert_list(np.nonzero(flags)[0])
+        visits = sg.DeviceArray(np.zeros(n, np.uint32))
+        ops.advance.frontier(G, fin, fout, ops.OP_COUNT_VISITS, ops.op_args([visits]), direction, lb, expected_size=1)
+        if direction == 0:
+            want = np.where(flags, g.degrees(), 0)
+        else:
+            want = np.array([0 if flags[v] else int(flags[col[ro[v]:ro[v + 1]]].sum()) for v in range(n)])
+        assert np.array_equal(visits.numpy(), want)
+        assert np.array_equal(fout.flags(), reference_advance(ro, col, flags, direction))
